@@ -94,6 +94,14 @@ bool device_loop_default() {
 
 constexpr uint64_t kSegsPerShard = 256;
 
+// Count-only joins: tables of at least kPivotMinRows rows send the rows of
+// lists of at least kPivotMinLen values to the pivot kernel.  The line for the
+// lists is measured beside the kernel; below about a million rows (an R-MAT
+// triangle of scale 16) its launches, two more scans and one block per SM
+// leave nothing to gain.
+constexpr uint64_t kPivotMinRows = 1 << 20;
+constexpr int64_t kPivotMinLen = 256;
+
 PipePlan Database::plan_pipeline(const Op& op, bool recursive, uint64_t iteration,
                                  const std::map<std::string, TrieView>* dviews) {
   std::map<std::string, int> slot;
@@ -357,21 +365,20 @@ void Database::exec_pipeline(const Op& op, bool recursive, uint64_t iteration) {
     DevBuf wscr(join_work_scratch_bytes(cur.n), L_.stream);
     Scratch s{wscr.as<char>(), wscr.bytes(), 0};
     size_t pid = prof_begin("join_count");
-    // the last level of a count-only rule: rows probing a long bitmapped
-    // list of the table's first column go to the pivot kernel (join.cu)
+    // the last level of a count-only rule: rows probing a long list of the
+    // table's first column go to the pivot kernel (join.cu)
     lv.pivot_src = -1;
-    if (last && op.count && opt_pivot_min_ > 0 && !(sharded && op.shard == Op::Work) &&
+    const int64_t pivot_min = opt_pivot_min_ >= 0 ? opt_pivot_min_ : cur.n >= kPivotMinRows ? kPivotMinLen : 0;
+    if (last && op.count && pivot_min > 0 && !(sharded && op.shard == Op::Work) &&
         !group_bounds_.count(op.rule) && lv.kind == kColumnJoin && lv.nsrc == 2 && lv.nfilt == 0 &&
         !lv.wide && cur.n > 0) {
       for (int ps = 0; ps < 2; ps++) {
         const SrcSpec& P = lv.src[ps];
         const SrcSpec& D = lv.src[1 - ps];
-        if (P.prefix_slot == 0 && D.prefix_slot != 0 && P.mode == kSrcPlain && D.mode == kSrcPlain &&
-            P.t.bdir && P.t.bpool && P.t.bwords && P.t.bslots && P.t.dir_n &&
-            join_pivot_smem_bytes(P.t.bwords) <= kPivotSmemMax) {
+        if (P.prefix_slot == 0 && D.prefix_slot != 0 && P.mode == kSrcPlain && D.mode == kSrcPlain && P.t.dir &&
+            P.t.dir_n > 1 && join_pivot_smem_bytes(P.t.dir_n) <= kPivotSmemMax) {
           lv.pivot_src = ps;
-          lv.pivot_min = (uint32_t)std::min<int64_t>(opt_pivot_min_, 0xffffffffll);
-          lv.pivot_slots = P.t.bslots;
+          lv.pivot_min = (uint32_t)std::min<int64_t>(pivot_min, 0xffffffffll);
           break;
         }
       }
@@ -397,7 +404,7 @@ void Database::exec_pipeline(const Op& op, bool recursive, uint64_t iteration) {
       total = seg_owned(total, lv.seg, shard_world_, shard_rank_);
     }
     // the expand pass's own scratch, sized for this level's candidates
-    DevBuf xscr(join_expand_scratch_bytes(L_, total) + (w.poffs ? join_pivot_scratch_bytes(lv.pivot_slots) : 0),
+    DevBuf xscr(join_expand_scratch_bytes(L_, total) + (w.poffs ? join_pivot_scratch_bytes(lv) : 0),
                 L_.stream);
     Scratch xs{xscr.as<char>(), xscr.bytes(), 0};
     if (last) {

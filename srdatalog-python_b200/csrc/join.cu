@@ -34,6 +34,8 @@ namespace srdl {
 
 constexpr int kJThreads = 256;
 constexpr uint32_t kNoPair = 0xffffffffu;
+// Pivot rows: the driving list is at most this many times the pivot's list.
+constexpr uint32_t kPvRatio = 3;
 
 // Position of the pair (a, b) in a pair index (a binary view whose row
 // positions number the pairs), or kNoPair.
@@ -123,7 +125,16 @@ __global__ void __launch_bounds__(kJThreads) join_count_kernel(LevelSpec lv, Tab
       src_list(lv.src[1], in, r, b1, n1);
       const uint32_t* v0 = lv.src[0].prefix_slot < 0 ? lv.src[0].t.roots : lv.src[0].t.lo;
       const uint32_t* v1 = lv.src[1].prefix_slot < 0 ? lv.src[1].t.roots : lv.src[1].t.lo;
-      const int bd = n1 < n0 ? 1 : 0;
+      int bd = n1 < n0 ? 1 : 0;
+      // a pivot row: the pivot source's list is long enough to be held as a
+      // bitmap by the pivot kernel, and the other list, which then drives, is
+      // at most kPvRatio times as long
+      bool piv = false;
+      if (pwork) {
+        const uint32_t np = lv.pivot_src == 0 ? n0 : n1, nd = lv.pivot_src == 0 ? n1 : n0;
+        piv = np >= lv.pivot_min && nd <= (uint64_t)kPvRatio * np;
+        if (piv) bd = 1 - lv.pivot_src;
+      }
       const uint32_t* dv = bd ? v1 : v0;
       const uint32_t* ov = bd ? v0 : v1;
       uint32_t db = bd ? b1 : b0, de = db + (bd ? n1 : n0);
@@ -135,7 +146,8 @@ __global__ void __launch_bounds__(kJThreads) join_count_kernel(LevelSpec lv, Tab
       } else {
         de = db;
       }
-      work[r] = de - db;
+      work[r] = piv ? 0 : de - db;
+      if (pwork) pwork[r] = piv ? (uint64_t)(de - db) : 0;
       drv[r] = (uint8_t)bd;
       beg[r] = db;
       orange[r] = make_uint2(ob, oe);
@@ -144,14 +156,6 @@ __global__ void __launch_bounds__(kJThreads) join_count_kernel(LevelSpec lv, Tab
         const uint32_t* obd = bd ? lv.src[0].t.bdir : lv.src[1].t.bdir;
         const int ops = bd ? lv.src[0].prefix_slot : lv.src[1].prefix_slot;
         obm[r] = (obd && ops >= 0) ? obd[in.col[ops][r]] : kNoBitmap;
-        if (pwork) {
-          // a pivot row: the probed list is the pivot source's, bitmapped
-          // and long; its candidates move from cj2 to the pivot kernel
-          const bool piv = bd != lv.pivot_src && obm[r] != kNoBitmap &&
-                           (lv.pivot_src == 0 ? n0 : n1) >= lv.pivot_min;
-          pwork[r] = piv ? (uint64_t)(de - db) : 0;
-          if (piv) work[r] = 0;
-        }
       }
     } else if (lv.kind == kColumnJoin) {
       uint32_t best = 0xffffffffu, bb = 0;
@@ -838,17 +842,39 @@ static int cj2_blocks_per_sm(bool seg, int emit) {
 //
 // Count-only two-source column join, pivot rows only (join_count marks them):
 // rows (a, ...) whose driver list is the other source's and whose probed
-// list is a's, a long list with a bitmap.  Rows are sorted by a, so the
-// pivot rows of one a form a run: pivot_runs_kernel finds every bitmapped
-// value's run (two binary searches in the table's first column, one thread
-// per value) and splits it into pieces of kPvPiece candidates.  A block (one
-// per SM, 1024 threads) takes pieces in order from a device counter, copies
-// the piece's bitmap into shared memory (again only when the value changes),
-// and its 32 warps walk the piece's candidates as the cj2 kernel does, each
-// candidate a bit test in shared memory instead of a probe of the bitmap in
-// global memory.
+// list is a's.  Rows are sorted by a, so the pivot rows of one a form a run:
+// pivot_runs_kernel finds the run of every value with a long enough list (two
+// binary searches in the table's first column, one thread per value) and
+// splits it into pieces of about kPvPiece candidates, a row belonging to the
+// piece it starts in.  A block (one per SM, 1024 threads) takes pieces from a
+// device counter, sets the bits of a's list in a shared-memory bitmap of the
+// whole value domain and tests every candidate against it.
+//
+// Bound: a candidate costs its own four bytes (read through L2 in 16-byte
+// loads), one shared-memory word and about nine integer operations; probing a
+// bitmap in global memory instead costs a sector per candidate and the L1 tag
+// stage (one line per cycle for a gather), which is what bounds
+// join_cj2_kernel.  The bitmap's words are spread over the banks by folding the
+// higher bits of a word's index into its lowest five: graph ids are far from
+// uniform in single bits (R-MAT's are 0 three times out of four), and without
+// the fold a lookup took eight wavefronts.  1,024 rows at a time are staged in
+// shared memory, one per thread: the thread tests the up to six candidates that
+// share a 16-byte quad with another row itself, the whole quads between them are
+// numbered by one block scan, and warps take 512 quads at a time, so short rows
+// and a hub's long ones cost the same per candidate and no lane idles.  A lane
+// finds its first quad's row by binary search in shared memory and steps forward
+// from there, four loads in flight.  The next piece is looked up while the
+// current one is counted.
+//
+// R-MAT scale 20 triangle (3.0e9 candidates if the shorter list always drives):
+// the level took 7.64 ms on join_cj2_kernel alone and takes 5.08 ms with the
+// pivot rows here (3.2 ms) and the rest there (1.9 ms).  Lists from 96 values
+// on instead of 256 cost 0.2 ms more (a bitmap is cleared and filled per
+// list), a driving list of at most 1 or 6 times the pivot's instead of 3 cost
+// 0.37 and 0.06 ms more.
 constexpr int kPvThreads = 1024;
 constexpr uint64_t kPvPiece = 1u << 19;  // candidates per piece
+constexpr uint32_t kPvQuads = 512;       // 16-byte quads a warp takes at a time
 
 // First i in [lo, hi) with a[i] >= x (a sorted).
 __device__ __forceinline__ uint64_t pv_lower(const uint32_t* a, uint64_t lo, uint64_t hi, uint32_t x) {
@@ -860,109 +886,180 @@ __device__ __forceinline__ uint64_t pv_lower(const uint32_t* a, uint64_t lo, uin
   return lo;
 }
 
-// Per bitmap slot (a bitmapped value v): the rows of v in the table (first
-// column pcol, true row count min(cap, *d_n)), their pivot candidates
-// [cand_lo, cand_hi) and the number of pieces they make.
-__global__ void pivot_runs_kernel(const uint32_t* __restrict__ bdir, uint32_t nv, const uint32_t* __restrict__ pcol,
-                                  uint64_t cap, const uint64_t* __restrict__ d_n, const uint64_t* __restrict__ poffs,
-                                  uint32_t nslots, uint64_t* __restrict__ run_lo, uint64_t* __restrict__ run_hi,
-                                  uint64_t* __restrict__ cand_lo, uint64_t* __restrict__ cand_hi,
+// A run of pivot rows: the rows [row_lo, row_hi) of one first-column value,
+// their candidates [cand_lo, cand_hi) in poffs.
+struct PvRun {
+  uint64_t row_lo, row_hi, cand_lo, cand_hi;
+  uint32_t val, pad;
+};
+
+// Every value v whose list in the pivot source has at least min_len entries
+// takes a run slot; pieces[slot] = the pieces its candidates make.  The table's
+// true row count is min(cap, *d_n).  At most max_runs values qualify (the
+// caller's bound: rows of the index / min_len).
+__global__ void pivot_runs_kernel(const uint32_t* __restrict__ dir, uint32_t nv, uint32_t min_len,
+                                  const uint32_t* __restrict__ pcol, uint64_t cap, const uint64_t* __restrict__ d_n,
+                                  const uint64_t* __restrict__ poffs, uint32_t max_runs,
+                                  unsigned int* __restrict__ d_runs, PvRun* __restrict__ runs,
                                   uint64_t* __restrict__ pieces) {
   const uint64_t nrows = dev_size(cap, d_n);
   for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
-    const uint32_t slot = bdir[v];
-    if (slot == kNoBitmap || slot >= nslots) continue;
+    if (dir[v + 1] - dir[v] < min_len) continue;
     const uint64_t lo = pv_lower(pcol, 0, nrows, v);
     const uint64_t hi = pv_lower(pcol, lo, nrows, v + 1);
     const uint64_t cl = poffs[lo], ch = poffs[hi];
-    run_lo[slot] = lo;
-    run_hi[slot] = hi;
-    cand_lo[slot] = cl;
-    cand_hi[slot] = ch;
+    if (cl == ch) continue;
+    const unsigned int slot = atomicAdd(d_runs, 1u);
+    if (slot >= max_runs) continue;
+    runs[slot] = PvRun{lo, hi, cl, ch, v, 0};
     pieces[slot] = (ch - cl + kPvPiece - 1) / kPvPiece;
   }
 }
 
+// Place of value v's word in the bitmap (blocks of 32 words are permuted).
+__device__ __forceinline__ uint32_t pv_place(uint32_t v) {
+  return (v >> 5) ^ (((v >> 10) ^ (v >> 15)) & 31u);
+}
+__device__ __forceinline__ uint32_t pv_test(const uint32_t* bm, uint32_t v) {
+  return (bm[pv_place(v)] >> (v & 31)) & 1u;
+}
+
+// dvals: the driving lists (16-byte aligned); pvals / pdir: the pivot source's
+// lists.
 __global__ void __launch_bounds__(kPvThreads, 1) join_pivot_count_kernel(
     const uint32_t* __restrict__ dvals, const uint64_t* __restrict__ poffs, const uint32_t* __restrict__ beg,
-    const uint64_t* __restrict__ run_lo, const uint64_t* __restrict__ run_hi,
-    const uint64_t* __restrict__ cand_lo, const uint64_t* __restrict__ cand_hi,
-    const uint64_t* __restrict__ piece_offs, uint32_t nslots, const uint32_t* __restrict__ bpool,
+    const uint32_t* __restrict__ pvals, const uint32_t* __restrict__ pdir, const PvRun* __restrict__ runs,
+    const uint64_t* __restrict__ piece_offs, const unsigned int* __restrict__ d_runs, uint32_t max_runs,
     uint32_t bwords, unsigned long long* __restrict__ queue, unsigned long long* __restrict__ d_out_n) {
   extern __shared__ __align__(16) uint32_t bm[];
-  __shared__ uint64_t s_c0, s_c1, s_rl, s_rh;
-  __shared__ uint32_t s_slot;
-  __shared__ int s_done;
+  struct Piece {
+    uint64_t c0, c1;  // candidates
+    uint64_t r0, r1;  // rows: of c0, and past that of c1 - 1
+    uint32_t val;
+    int done;
+  };
+  __shared__ Piece pc[2];
+  __shared__ unsigned int s_next;         // next quads to take
+  __shared__ uint32_t s_inc[kPvThreads];  // staged rows: quads up to and including the row's
+  __shared__ uint32_t s_base[kPvThreads]; // s_base + (quad number) = quad of dvals
+  __shared__ uint32_t scan_sh[kPvThreads / 32 + 1];
   __shared__ unsigned long long s_sum[kPvThreads / 32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const uint64_t npieces = piece_offs[nslots];
-  uint32_t loaded = kNoBitmap;
+  const uint32_t nruns = min(*d_runs, max_runs);
+  const uint64_t npieces = piece_offs[max_runs];
+  // Takes the next piece from the queue (whole warp).
+  auto fetch = [&](Piece& p) {
+    unsigned long long k = 0;
+    if (lane == 0) k = atomicAdd(queue, 1ull);
+    k = __shfl_sync(kAllLanes, k, 0);
+    if (k >= npieces) {
+      if (lane == 0) p.done = 1;
+      return;
+    }
+    // the run of piece k: the last one with piece_offs[run] <= k
+    const uint64_t u = warp_partition_point(0, nruns, [&](uint64_t i) { return piece_offs[i] <= k; }) - 1;
+    const PvRun rn = runs[u];
+    const uint64_t c0 = rn.cand_lo + (k - piece_offs[u]) * kPvPiece;
+    const uint64_t c1 = c0 + kPvPiece < rn.cand_hi ? c0 + kPvPiece : rn.cand_hi;
+    const uint64_t r0 = warp_partition_point(rn.row_lo, rn.row_hi, [&](uint64_t i) { return poffs[i] <= c0; }) - 1;
+    uint64_t r1 = rn.row_hi;
+    if (c1 < rn.cand_hi) r1 = warp_partition_point(r0, rn.row_hi, [&](uint64_t i) { return poffs[i] < c1; });
+    if (lane == 0) {
+      p.c0 = c0;
+      p.c1 = c1;
+      p.r0 = r0;
+      p.r1 = r1;
+      p.val = rn.val;
+      p.done = 0;
+    }
+  };
   unsigned long long counted = 0;
-  for (;;) {
-    if (threadIdx.x == 0) {
-      const unsigned long long k = atomicAdd(queue, 1ull);
-      s_done = k >= npieces;
-      if (k < npieces) {
-        // the slot of piece k: the last slot with piece_offs[slot] <= k
-        uint32_t lo = 0, hi = nslots;
-        while (hi - lo > 1) {
-          const uint32_t m = lo + (hi - lo) / 2;
-          if (piece_offs[m] <= k) lo = m;
-          else hi = m;
-        }
-        const uint64_t j = k - piece_offs[lo];
-        const uint64_t c0 = cand_lo[lo] + j * kPvPiece;
-        s_slot = lo;
-        s_c0 = c0;
-        s_c1 = c0 + kPvPiece < cand_hi[lo] ? c0 + kPvPiece : cand_hi[lo];
-        s_rl = run_lo[lo];
-        s_rh = run_hi[lo];
-      }
-    }
+  uint32_t held = 0xffffffffu;  // value whose bitmap is in shared memory
+  if (wid == 0) fetch(pc[0]);
+  for (int cur = 0;; cur ^= 1) {
     __syncthreads();
-    if (s_done) break;
-    const uint32_t slot = s_slot;
-    const uint64_t c0 = s_c0, c1 = s_c1, rl = s_rl, rh = s_rh;
-    if (slot != loaded) {
-      // (word loads: a bitmap starts at slot * bwords words, not always on
-      // a 16-byte boundary)
-      const uint32_t* src = bpool + (uint64_t)slot * bwords;
-      for (uint32_t i = threadIdx.x; i < bwords; i += kPvThreads) bm[i] = src[i];
+    if (pc[cur].done) break;
+    const uint64_t c0 = pc[cur].c0, c1 = pc[cur].c1, r0 = pc[cur].r0, r1 = pc[cur].r1;
+    const uint32_t val = pc[cur].val;
+    if (val != held) {
+      uint4* z = reinterpret_cast<uint4*>(bm);
+      for (uint32_t i = threadIdx.x; i < bwords / 4; i += kPvThreads) z[i] = make_uint4(0, 0, 0, 0);
       __syncthreads();
-      loaded = slot;
-    }
-    // warp wid walks its share of the piece in rounds of 32 candidates; the
-    // row of the round's first candidate is kept while the warp stays in it
-    const uint64_t len = c1 - c0;
-    const uint64_t wb = c0 + len * wid / (kPvThreads / 32);
-    const uint64_t we = c0 + len * (wid + 1) / (kPvThreads / 32);
-    if (wb < we) {
-      uint64_t r0 = warp_partition_point(rl, rh, [&](uint64_t i) { return poffs[i] <= wb; }) - 1;
-      uint64_t crow = ~0ull, c_off = 0, c_end = 0;
-      uint32_t cbeg = 0;
-      for (uint64_t base = wb; base < we; base += 32) {
-        const uint64_t w = base + lane;
-        const bool ok = w < we;
-        if (r0 != crow) {
-          crow = r0;
-          c_off = poffs[r0];
-          c_end = poffs[r0 + 1];
-          cbeg = beg[r0];
-        }
-        uint32_t v = 0;
-        if (base + 31 < c_end) {
-          if (ok) v = dvals[cbeg + (uint32_t)(w - c_off)];
-        } else if (ok) {
-          const uint64_t r = gallop_row(poffs, r0, rh, w);
-          v = dvals[beg[r] + (uint32_t)(w - poffs[r])];
-        }
-        if (ok) counted += (bm[v >> 5] >> (v & 31)) & 1u;
-        // the next round's first row (the row of its first candidate)
-        const uint64_t nb = base + 32;
-        if (nb < we && nb >= c_end) r0 = gallop_row(poffs, r0, rh, nb);
+      const uint32_t pe = pdir[val + 1];
+      for (uint32_t i = pdir[val] + threadIdx.x; i < pe; i += kPvThreads) {
+        const uint32_t v = pvals[i];
+        atomicOr(&bm[pv_place(v)], 1u << (v & 31));
       }
+      held = val;
+      __syncthreads();
     }
-    __syncthreads();  // (the bitmap and s_* are rewritten by the next piece)
+    const uint4* src = reinterpret_cast<const uint4*>(dvals);
+    for (uint64_t rb = r0; rb < r1; rb += kPvThreads) {
+      // this thread's row: its candidates of the piece, [b, e) in dvals
+      uint32_t b = 0, e = 0;
+      const uint64_t row = rb + threadIdx.x;
+      if (row < r1) {
+        const uint64_t ro = poffs[row], re = poffs[row + 1];
+        const uint64_t from = ro > c0 ? ro : c0, to = re < c1 ? re : c1;
+        if (from < to) {
+          b = beg[row] + (uint32_t)(from - ro);
+          e = b + (uint32_t)(to - from);
+        }
+      }
+      // whole quads [qa, qb); the candidates before and after them are this
+      // thread's
+      const uint32_t qa = (b + 3) / 4, qb = e / 4;
+      const uint32_t m = qb > qa ? qb - qa : 0;
+      uint32_t quads;
+      const uint32_t ex = block_excl_scan(m, scan_sh, &quads);
+      s_inc[threadIdx.x] = ex + m;
+      s_base[threadIdx.x] = qa - ex;
+      {
+        const uint32_t h1 = 4 * qa < e ? 4 * qa : e, t0 = 4 * qb > h1 ? 4 * qb : h1;
+        uint32_t n = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < 3; k++) {
+          if (b + k < h1) n += pv_test(bm, __ldg(dvals + b + k));
+          if (t0 + k < e) n += pv_test(bm, __ldg(dvals + t0 + k));
+        }
+        counted += n;
+      }
+      if (threadIdx.x == 0) s_next = 0;
+      __syncthreads();
+      if (rb == r0 && wid == 0) fetch(pc[cur ^ 1]);
+      for (;;) {
+        uint32_t q0 = 0;
+        if (lane == 0) q0 = atomicAdd(&s_next, kPvQuads);
+        q0 = __shfl_sync(kAllLanes, q0, 0);
+        if (q0 >= quads) break;
+        const uint32_t q1 = q0 + kPvQuads < quads ? q0 + kPvQuads : quads;
+        // the row of this lane's first quad: the rows up to it come before
+        uint32_t r = 0;
+#pragma unroll
+        for (uint32_t d = kPvThreads / 2; d > 0; d >>= 1)
+          if (s_inc[r + d - 1] <= q0 + lane) r += d;
+        uint32_t n = 0;
+        uint32_t q = q0 + lane;
+        for (; q + 96 < q1; q += 128) {
+          uint4 x[4];
+#pragma unroll
+          for (int u = 0; u < 4; u++) {
+            while (s_inc[r] <= q + 32 * u) r++;
+            x[u] = __ldg(src + (s_base[r] + q + 32 * u));
+          }
+#pragma unroll
+          for (int u = 0; u < 4; u++)
+            n += pv_test(bm, x[u].x) + pv_test(bm, x[u].y) + pv_test(bm, x[u].z) + pv_test(bm, x[u].w);
+        }
+        for (; q < q1; q += 32) {
+          while (s_inc[r] <= q) r++;
+          const uint4 x = __ldg(src + (s_base[r] + q));
+          n += pv_test(bm, x.x) + pv_test(bm, x.y) + pv_test(bm, x.z) + pv_test(bm, x.w);
+        }
+        counted += n;
+      }
+      __syncthreads();  // (the staged rows are rewritten)
+    }
   }
   // block total -> the level's count
   const unsigned long long ws = warp_sum(counted);
@@ -985,7 +1082,7 @@ JoinWork join_count(const Launch& L, const LevelSpec& lv, const Table& in, Scrat
   if (lv.kind == kColumnJoin && lv.nsrc == 2 && !lv.wide && (lv.src[0].t.bdir || lv.src[1].t.bdir))
     w.obm = s.take<uint32_t>(in.n ? in.n : 1);
   uint64_t* pwork = nullptr;
-  if (w.obm && lv.pivot_src >= 0 && in.n) {
+  if (lv.pivot_src >= 0 && in.n) {
     pwork = s.take<uint64_t>(in.n);
     w.poffs = s.take<uint64_t>(in.n + 1);
   }
@@ -1000,46 +1097,50 @@ JoinWork join_count(const Launch& L, const LevelSpec& lv, const Table& in, Scrat
   return w;
 }
 
-size_t join_pivot_smem_bytes(uint32_t bwords) { return (size_t)bwords * 4; }
+// Words of a bitmap over the values a dense directory of dir_n entries covers,
+// whole blocks of 32.
+static uint32_t pv_words(uint32_t dir_n) { return (uint32_t)((((uint64_t)dir_n + 31) / 32 + 31) & ~uint64_t(31)); }
 
-size_t join_pivot_scratch_bytes(uint32_t nslots) {
-  return 7 * ((size_t)(nslots + 1) * 8 + 511) + scan_scratch_bytes(nslots) + 2048;
+size_t join_pivot_smem_bytes(uint32_t dir_n) { return (size_t)pv_words(dir_n) * 4; }
+
+// Values of the pivot source whose lists reach pivot_min.
+static uint32_t pv_max_runs(const LevelSpec& lv) {
+  return (uint32_t)std::min<uint64_t>(lv.src[lv.pivot_src].t.n / lv.pivot_min + 1, 0xfffffffeull);
 }
 
-// The pivot rows' count (count mode; w.poffs set): the runs of the
-// bitmapped values, their pieces, then one block per SM over the pieces.
+size_t join_pivot_scratch_bytes(const LevelSpec& lv) {
+  const size_t m = (size_t)pv_max_runs(lv) + 1;
+  return m * (sizeof(PvRun) + 16) + scan_scratch_bytes(m) + 4096;
+}
+
+// The pivot rows' count (count mode; w.poffs set): the runs of the long
+// lists' values, their pieces, then one block per SM over the pieces.
 static void join_pivot_count(const Launch& L, const LevelSpec& lv, const Table& in, const JoinWork& w,
                              unsigned long long* d_out_n, Scratch& s) {
   const int ps = lv.pivot_src, ds = 1 - ps;
   const SrcSpec& P = lv.src[ps];
   const SrcSpec& D = lv.src[ds];
   const uint32_t* dvals = D.prefix_slot < 0 ? D.t.roots : D.t.lo;
-  const uint32_t nslots = lv.pivot_slots;
-  if (!nslots || !P.t.dir_n) return;
-  const size_t smem = join_pivot_smem_bytes(P.t.bwords);
-  static size_t attr = 0;
-  if (smem > attr) {
-    SRDL_CUDA(cudaFuncSetAttribute(join_pivot_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)smem));
-    attr = smem;
-  }
-  uint64_t* run_lo = s.take<uint64_t>(nslots);
-  uint64_t* run_hi = s.take<uint64_t>(nslots);
-  uint64_t* cand_lo = s.take<uint64_t>(nslots);
-  uint64_t* cand_hi = s.take<uint64_t>(nslots);
-  uint64_t* pieces = s.take<uint64_t>(nslots);
-  uint64_t* piece_offs = s.take<uint64_t>(nslots + 1);
-  unsigned long long* q = s.take<unsigned long long>(1);
-  SRDL_CUDA(cudaMemsetAsync(pieces, 0, nslots * 8, L.stream));
-  SRDL_CUDA(cudaMemsetAsync(q, 0, sizeof(unsigned long long), L.stream));
+  if (P.t.dir_n < 2) return;
+  const size_t smem = join_pivot_smem_bytes(P.t.dir_n);
+  // (the attribute is per device and only ever the largest: set on each call)
+  SRDL_CUDA(cudaFuncSetAttribute(join_pivot_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)kPivotSmemMax));
+  const uint32_t max_runs = pv_max_runs(lv);
+  PvRun* runs = s.take<PvRun>(max_runs);
+  uint64_t* pieces = s.take<uint64_t>(max_runs);
+  uint64_t* piece_offs = s.take<uint64_t>((size_t)max_runs + 1);
+  unsigned long long* q = s.take<unsigned long long>(2);  // piece queue, run count
+  unsigned int* d_runs = reinterpret_cast<unsigned int*>(q + 1);
+  SRDL_CUDA(cudaMemsetAsync(pieces, 0, (size_t)max_runs * 8, L.stream));
+  SRDL_CUDA(cudaMemsetAsync(q, 0, 2 * sizeof(unsigned long long), L.stream));
   const uint32_t nv = P.t.dir_n - 1;
-  pivot_runs_kernel<<<(int)std::min<uint64_t>((nv + 255) / 256, (uint64_t)L.num_sms * 8), 256, 0, L.stream>>>(
-      P.t.bdir, nv, in.col[P.prefix_slot], in.n, in.d_n, w.poffs, nslots, run_lo, run_hi, cand_lo, cand_hi,
-      pieces);
-  exclusive_scan_u64(L, pieces, nslots, piece_offs, s);
+  pivot_runs_kernel<<<(int)std::min<uint64_t>(((uint64_t)nv + 255) / 256, (uint64_t)L.num_sms * 8), 256, 0,
+                      L.stream>>>(P.t.dir, nv, lv.pivot_min, in.col[P.prefix_slot], in.n, in.d_n, w.poffs, max_runs,
+                                  d_runs, runs, pieces);
+  exclusive_scan_u64(L, pieces, max_runs, piece_offs, s);
   join_pivot_count_kernel<<<L.num_sms, kPvThreads, smem, L.stream>>>(
-      dvals, w.poffs, w.beg, run_lo, run_hi, cand_lo, cand_hi, piece_offs, nslots, P.t.bpool, P.t.bwords, q,
-      d_out_n);
+      dvals, w.poffs, w.beg, P.t.lo, P.t.dir, runs, piece_offs, d_runs, max_runs, pv_words(P.t.dir_n), q, d_out_n);
   SRDL_CUDA(cudaGetLastError());
   count_launches(2);
 }

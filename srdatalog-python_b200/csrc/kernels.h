@@ -247,14 +247,13 @@ struct LevelSpec {
   const uint32_t* grp_bounds = nullptr;  // n_groups + 1 sorted entries
   uint32_t n_groups = 0;
   unsigned long long* grp_counts = nullptr;
-  // Count-only two-source column joins: rows whose driver is the other
-  // source's list and whose probed list -- source pivot_src's, indexed by
-  // the table's first (sorted) column -- has a bitmap and at least
-  // pivot_min values are counted by the pivot kernel (the bitmap of the
-  // rows' common first value held in shared memory) instead of cj2.
+  // Count-only two-source column joins: rows whose list in source pivot_src
+  // -- indexed by the table's first (sorted) column -- has at least pivot_min
+  // (> 0) values and is not far shorter than the other list are counted by
+  // the pivot kernel (that list's bitmap held in shared memory, the other
+  // list driving) instead of cj2.
   int pivot_src = -1;
   uint32_t pivot_min = 0;
-  uint32_t pivot_slots = 0;  // bitmaps of the pivot source
   // Sharded work: expand only segments seg_rank, seg_rank + seg_world, ...
   // of `seg` work items each (seg a multiple of 32; 0: every item).
   uint64_t seg = 0;
@@ -282,11 +281,12 @@ struct JoinWork {
 };
 JoinWork join_count(const Launch& L, const LevelSpec& lv, const Table& in, Scratch& s);
 
-// Shared memory the pivot kernel needs for one bitmap of `bwords` words;
-// levels whose bitmaps need more than kPivotSmemMax keep the cj2 kernel.
-size_t join_pivot_smem_bytes(uint32_t bwords);
+// Shared memory the pivot kernel needs for a bitmap of the values that a dense
+// directory of dir_n entries covers; levels that need more than kPivotSmemMax
+// keep the cj2 kernel.
+size_t join_pivot_smem_bytes(uint32_t dir_n);
 // Scratch the pivot pass adds to a level's expand scratch.
-size_t join_pivot_scratch_bytes(uint32_t nslots);
+size_t join_pivot_scratch_bytes(const LevelSpec& lv);
 constexpr size_t kPivotSmemMax = 200 * 1024;
 
 // Pass 2: expands `total` work items (all of the count pass's items, or

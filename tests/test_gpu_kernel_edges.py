@@ -1,0 +1,43 @@
+'''Sizes at which a kernel or the rule that picks it can go wrong: edges of
+tiles and blocks, remainders, the smallest and the largest of a range.  Every
+result is exact, against the oracle's restatement.'''
+
+import numpy as np
+import oracle
+import pytest
+from conftest import load_plan
+from srdatalog_b200 import native
+from srdatalog_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip('torch')
+
+
+@pytest.mark.parametrize('pivot_min', [1, 3, 64, 1 << 20])
+@pytest.mark.parametrize('scale,draws', [(6, 3000), (12, 60_000)])
+def test_pivot_rows_of_every_length(scale, draws, pivot_min):
+  '''Count by shared-memory bitmaps: lists of any length, hubs that share their
+  candidates among warps, and none at all.'''
+  e = W.rmat_edges(scale, draws, seed=scale)
+  with native.Database(load_plan('triangle')) as db:
+    db.set_option('pivot_min', pivot_min)
+    db.load_rows('KnowsInput', e)
+    db.run()
+    assert db.count('TriangleJoin') == oracle.triangle_count(e)
+
+
+def test_pivot_hub_of_many_pieces():
+  '''One value whose rows make several million candidates.'''
+  hub = np.stack([np.zeros(5000, np.uint32), np.arange(1, 5001, dtype=np.uint32)], 1)
+  rng = np.random.default_rng(3)
+  rest = rng.integers(1, 5001, (900_000, 2)).astype(np.uint32)
+  rest = rest[rest[:, 0] < rest[:, 1]]
+  e = np.unique(np.concatenate([hub, rest]), axis=0)
+  counts = []
+  for pm in (0, 16):
+    with native.Database(load_plan('triangle')) as db:
+      db.set_option('pivot_min', pm)
+      db.load_rows('KnowsInput', e)
+      db.run()
+      counts.append(db.count('TriangleJoin'))
+  assert counts[0] == counts[1] == oracle.triangle_count(e)
