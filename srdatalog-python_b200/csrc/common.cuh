@@ -237,6 +237,43 @@ __device__ __forceinline__ T block_excl_scan(T v, T* sh, T* total) {
   return r;
 }
 
+// Sum of a[0..k), in every thread of the block (sh as for block_excl_scan).
+template <typename T>
+__device__ __forceinline__ uint64_t block_prefix(const T* a, uint32_t k, uint64_t* sh) {
+  uint64_t s = 0;
+  for (uint32_t i = threadIdx.x; i < k; i += blockDim.x) s += a[i];
+  uint64_t tot;
+  block_excl_scan(s, sh, &tot);
+  return tot;
+}
+
+// Exclusive scan of in[0..n) into out[0..n) by one block of THREADS threads;
+// returns the total.  in and out may be the same array.
+template <int THREADS>
+__device__ __forceinline__ uint64_t block_scan_write(const uint64_t* in, uint32_t n, uint64_t* out, uint64_t* sh) {
+  constexpr int kItems = 4;
+  uint64_t base = 0;
+  for (uint32_t tile = 0; tile < n; tile += THREADS * kItems) {
+    const uint32_t i0 = tile + threadIdx.x * kItems;
+    uint64_t v[kItems];
+    uint64_t s = 0;
+#pragma unroll
+    for (int j = 0; j < kItems; j++) {
+      v[j] = i0 + j < n ? in[i0 + j] : 0;
+      s += v[j];
+    }
+    uint64_t tot;
+    uint64_t run = base + block_excl_scan(s, sh, &tot);
+#pragma unroll
+    for (int j = 0; j < kItems; j++) {
+      if (i0 + j < n) out[i0 + j] = run;
+      run += v[j];
+    }
+    base += tot;
+  }
+  return base;
+}
+
 // First i in [lo, hi) where pred(i) is false, for a predicate that is true
 // on a prefix; called by all 32 lanes of a warp.  Each round tests 32 evenly
 // spaced positions, so the number of dependent load rounds is log32(hi-lo).

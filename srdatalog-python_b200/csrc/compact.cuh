@@ -1,15 +1,17 @@
-// compact.cuh -- order-preserving stream compaction in three launches.
+// compact.cuh -- order-preserving stream compaction in two launches.
 //
 //   1. flag   : each block owns a contiguous chunk; every warp evaluates the
 //               selector on 32 consecutive elements at a time and stores the
 //               ballot as one flag word (bit l = element 32w + l); the block's
 //               selected count goes to blk_counts;
-//   2. scan   : one block turns the per-block counts into offsets + total;
-//   3. write  : each block walks its chunk a 2048-element tile at a time;
-//               warp w takes the tile's elements [256w, 256w + 256) in eight
-//               rounds of 32, so a round's output positions are the running
-//               count plus the popcount of the lower lanes of its flag word:
-//               loads and stores are coalesced.
+//   2. write  : each block adds up the counts of the blocks before it (at
+//               most 8 per SM: a few loads per thread, cheaper than a launch
+//               that scans them), then walks its chunk a 2048-element tile
+//               at a time; warp w takes the tile's elements
+//               [256w, 256w + 256) in eight rounds of 32, so a round's output
+//               positions are the running count plus the popcount of the
+//               lower lanes of its flag word: loads and stores are coalesced.
+//               The last block writes the total.
 // No block waits on another, so nothing can spin.  Selectors provide
 //   __device__ void block_setup(uint64_t begin, uint64_t end);  (all threads)
 //   __device__ bool select(uint64_t i);
@@ -39,6 +41,12 @@ inline uint64_t cp_chunk(uint64_t n, int sms) {
 inline int cp_blocks(uint64_t n, uint64_t chunk) {
   uint64_t nb = (n + chunk - 1) / chunk;
   return nb ? (int)nb : 1;
+}
+// The same split with n known only on the device: nb blocks, whole tiles.
+__device__ __forceinline__ uint64_t cp_even_chunk(uint64_t n, uint64_t nb) {
+  const uint64_t tiles = (n + kCpTile - 1) / kCpTile;
+  const uint64_t per = (tiles + nb - 1) / nb;
+  return (per ? per : 1) * (uint64_t)kCpTile;
 }
 inline uint64_t cp_words(uint64_t n) { return (n + 31) / 32; }
 inline size_t cp_scratch_bytes(uint64_t n) {
@@ -80,23 +88,22 @@ __global__ void __launch_bounds__(kCpThreads) cp_flag_kernel(Sel sel, uint64_t n
   if (threadIdx.x == 0) blk_counts[blockIdx.x] = tot;
 }
 
-// One block; exclusive scan of nb block counts into offs[0..nb], total -> *d_total.
-__global__ void cp_scan_kernel(const uint32_t* blk_counts, int nb, uint64_t* offs,
-                               uint64_t* d_total);
-
 template <class Sel>
 __global__ void __launch_bounds__(kCpThreads) cp_write_kernel(Sel sel, uint64_t n, uint64_t chunk,
                                                               const uint32_t* __restrict__ flags,
-                                                              const uint64_t* offs,
+                                                              const uint32_t* __restrict__ blk_counts,
+                                                              uint64_t* d_total,
                                                               const uint64_t* d_n) {
   __shared__ uint32_t wtot[2][kCpWarps];
+  __shared__ uint64_t sh[kCpWarps + 1];
   n = dev_size(n, d_n);
   chunk = dev_chunk(chunk, n, kCpTile);
   const uint64_t begin = (uint64_t)blockIdx.x * chunk;
   const uint64_t end = begin + chunk < n ? begin + chunk : n;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const unsigned lt = lanemask_lt();
-  uint64_t base = offs[blockIdx.x];
+  uint64_t base = block_prefix(blk_counts, blockIdx.x, sh);
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *d_total = base + blk_counts[blockIdx.x];
   int par = 0;
   for (uint64_t tile = begin; tile < end; tile += kCpTile, par ^= 1) {
     // lane r < 8 fetches the flag word of round r of this warp's 256 elements
@@ -146,12 +153,10 @@ void compact(const Launch& L, Sel sel, uint64_t n, uint64_t* d_total, Scratch& s
   const uint64_t kchunk = d_n ? 0 : chunk;
   uint32_t* flags = s.take<uint32_t>(cp_words(n));
   uint32_t* counts = s.take<uint32_t>(nb);
-  uint64_t* offs = s.take<uint64_t>(nb + 1);
   cp_flag_kernel<Sel><<<nb, kCpThreads, 0, L.stream>>>(sel, n, kchunk, flags, counts, d_n);
-  cp_scan_kernel<<<1, 1024, 0, L.stream>>>(counts, nb, offs, d_total);
-  cp_write_kernel<Sel><<<nb, kCpThreads, 0, L.stream>>>(sel, n, kchunk, flags, offs, d_n);
+  cp_write_kernel<Sel><<<nb, kCpThreads, 0, L.stream>>>(sel, n, kchunk, flags, counts, d_total, d_n);
   SRDL_CUDA(cudaGetLastError());
-  count_launches(3);
+  count_launches(2);
 }
 
 // Keeps a[i] when it differs from a[i-1] (optional) and is absent from the
@@ -606,7 +611,6 @@ void compact_diff(const Launch& L, DedupDiffSel<K> sel, uint64_t n, uint64_t* d_
   const uint64_t tiles = (n + kCpTile - 1) / kCpTile;
   uint32_t* flags = s.take<uint32_t>(cp_words(n));
   uint32_t* counts = s.take<uint32_t>(nb);
-  uint64_t* offs = s.take<uint64_t>(nb + 1);
   if (sel.n_full <= kDmMaxFullRatio * n) {
     const uint64_t mtiles = (n + sel.n_full + kCpTile - 1) / kCpTile;
     SRDL_REQUIRE(mtiles < (1ull << 31), kErrCapacity, "set difference: too many rows");
@@ -620,11 +624,10 @@ void compact_diff(const Launch& L, DedupDiffSel<K> sel, uint64_t n, uint64_t* d_
     dm_mark_kernel<K><<<mgrid, kCpThreads, 0, L.stream>>>(sel, n, mtiles, split, mhpos, flags, nullptr,
                                                           kPathAny);
     cp_count_kernel<K><<<nb, kCpThreads, 0, L.stream>>>(flags, n, chunk, counts, sel, nullptr, kPathAny);
-    cp_scan_kernel<<<1, 1024, 0, L.stream>>>(counts, nb, offs, d_total);
-    cp_write_kernel<DedupDiffSel<K>><<<nb, kCpThreads, 0, L.stream>>>(sel, n, chunk, flags, offs,
-                                                                       nullptr);
+    cp_write_kernel<DedupDiffSel<K>><<<nb, kCpThreads, 0, L.stream>>>(sel, n, chunk, flags, counts,
+                                                                       d_total, nullptr);
     SRDL_CUDA(cudaGetLastError());
-    count_launches(5);
+    count_launches(4);
     return;
   }
   uint64_t* fpos = s.take<uint64_t>(tiles + 1);
@@ -635,11 +638,10 @@ void compact_diff(const Launch& L, DedupDiffSel<K> sel, uint64_t n, uint64_t* d_
                                                                                 hpos, nullptr, kPathAny);
   dd_flag_kernel<K><<<nb, kCpThreads, 0, L.stream>>>(sel, n, chunk, fpos, hpos, flags, counts,
                                                      nullptr, kPathAny);
-  cp_scan_kernel<<<1, 1024, 0, L.stream>>>(counts, nb, offs, d_total);
-  cp_write_kernel<DedupDiffSel<K>><<<nb, kCpThreads, 0, L.stream>>>(sel, n, chunk, flags, offs,
-                                                                     nullptr);
+  cp_write_kernel<DedupDiffSel<K>><<<nb, kCpThreads, 0, L.stream>>>(sel, n, chunk, flags, counts,
+                                                                     d_total, nullptr);
   SRDL_CUDA(cudaGetLastError());
-  count_launches(4);
+  count_launches(3);
 }
 
 // compact_diff with the key count on the device (device loop): `cap` keys
@@ -671,7 +673,6 @@ void compact_diff_dev(const Launch& L, DedupDiffSel<K> sel, uint64_t cap, const 
   const uint64_t mtiles = (cap + sel.n_full + kCpTile - 1) / kCpTile;
   uint32_t* flags = s.take<uint32_t>(cp_words(cap));
   uint32_t* counts = s.take<uint32_t>(nb);
-  uint64_t* offs = s.take<uint64_t>(nb + 1);
   uint64_t* fpos = s.take<uint64_t>(tiles + 1);
   uint64_t* split = s.take<uint64_t>(mtiles + 1);
   prefer_shared(dd_flag_kernel<K>);
@@ -690,11 +691,10 @@ void compact_diff_dev(const Launch& L, DedupDiffSel<K> sel, uint64_t cap, const 
                                                               kPathProbe);
   dd_flag_kernel<K><<<nb, kCpThreads, 0, L.stream>>>(sel, cap, 0, fpos, nullptr, flags, counts, d_n,
                                                      kPathProbe);
-  // either way: offsets and the ordered write of the kept keys
-  cp_scan_kernel<<<1, 1024, 0, L.stream>>>(counts, nb, offs, d_total);
-  cp_write_kernel<DedupDiffSel<K>><<<nb, kCpThreads, 0, L.stream>>>(sel, cap, 0, flags, offs, d_n);
+  // either way: the ordered write of the kept keys
+  cp_write_kernel<DedupDiffSel<K>><<<nb, kCpThreads, 0, L.stream>>>(sel, cap, 0, flags, counts, d_total, d_n);
   SRDL_CUDA(cudaGetLastError());
-  count_launches(7);
+  count_launches(6);
 }
 
 // Distinct first-column values of a sorted key array.

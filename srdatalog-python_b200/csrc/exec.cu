@@ -383,12 +383,9 @@ void Database::exec_pipeline(const Op& op, bool recursive, uint64_t iteration) {
         }
       }
     }
-    JoinWork w = join_count(L_, lv, cur, s);
+    // (the totals land in page-locked memory: nothing is copied back)
+    JoinWork w = join_count(L_, lv, cur, s, d_small_.as<uint64_t>() + 2, h_small_ + 3, h_small_ + 6);
     prof_end(pid, 8.0 * cur.n * (lv.n_in_slots + 3), (double)cur.n);
-    SRDL_CUDA(cudaMemcpyAsync(h_small_ + 3, w.offs + cur.n, 8, cudaMemcpyDeviceToHost, L_.stream));
-    if (w.poffs)
-      SRDL_CUDA(cudaMemcpyAsync(h_small_ + 6, w.poffs + cur.n, 8, cudaMemcpyDeviceToHost, L_.stream));
-    SRDL_CUDA(cudaMemsetAsync(d_small_.as<uint64_t>() + 2, 0, 8, L_.stream));
     SRDL_CUDA(cudaStreamSynchronize(L_.stream));
     uint64_t total = h_small_[3];
     const uint64_t pivot_total = w.poffs ? h_small_[6] : 0;  // the pivot kernel's candidates
@@ -492,7 +489,7 @@ void Database::exec_pipeline(const Op& op, bool recursive, uint64_t iteration) {
       // The table's row count stays on the device; the next level uses the
       // candidate total as capacity and reads the true count itself.
       DevBuf count(8, L_.stream);
-      SRDL_CUDA(cudaMemsetAsync(count.as<void>(), 0, 8, L_.stream));
+      if (!total) SRDL_CUDA(cudaMemsetAsync(count.as<void>(), 0, 8, L_.stream));
       pid = prof_begin("join_expand_table");
       join_expand(L_, lv, cur, w, total, &next, nullptr, count.as<uint64_t>(), xs);
       prof_end(pid, 4.0 * total * std::max(1, lv.nsrc), (double)total);

@@ -98,13 +98,31 @@ __device__ __forceinline__ bool src_contains(const SrcSpec& s, const Table& in, 
   return trie_child_contains(s.t, in.col[s.prefix_slot][r], v);
 }
 
-__global__ void __launch_bounds__(kJThreads) join_count_kernel(LevelSpec lv, Table in,
-                                                               uint64_t* __restrict__ work,
-                                                               uint8_t* __restrict__ drv,
-                                                               uint32_t* __restrict__ beg,
-                                                               uint2* __restrict__ orange,
-                                                               uint32_t* __restrict__ obm,
-                                                               uint64_t* __restrict__ pwork) {
+// Words a count launch sets: the chunk queues of the two-source join and a
+// counter of the caller's to zero, and where the totals of the offsets go
+// (device or page-locked host memory).
+struct CountInit {
+  unsigned long long* queue = nullptr;  // two words, zeroed
+  uint64_t* zero = nullptr;             // one word, zeroed
+  uint64_t* total = nullptr;            // SCAN: offs[in.n]
+  uint64_t* ptotal = nullptr;           // SCAN: poffs[in.n]
+};
+
+// Tables of at most this many rows are counted and scanned by one block in one
+// launch: up to four rows per thread, which costs less than the scan's launch.
+constexpr int kJSmallThreads = 1024;
+constexpr uint64_t kJSmallRows = 4096;
+
+// SCAN: a single block also turns work into offs (and pwork into poffs).
+template <bool SCAN>
+__global__ void __launch_bounds__(SCAN ? kJSmallThreads : kJThreads) join_count_kernel(
+    LevelSpec lv, Table in, uint64_t* work, uint8_t* __restrict__ drv, uint32_t* __restrict__ beg,
+    uint2* __restrict__ orange, uint32_t* __restrict__ obm, uint64_t* pwork, uint64_t* offs,
+    uint64_t* poffs, CountInit ci) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (ci.queue) ci.queue[0] = ci.queue[1] = 0;
+    if (ci.zero) *ci.zero = 0;
+  }
   // A table written by the previous level may fill only part of its
   // capacity; its true size is on the device and the rest expands to nothing.
   const uint64_t nrows = in.d_n ? min(in.n, *in.d_n) : in.n;
@@ -205,6 +223,22 @@ __global__ void __launch_bounds__(kJThreads) join_count_kernel(LevelSpec lv, Tab
         uint32_t b, e;
         trie_range(s.t, in.col[s.prefix_slot][r], b, e);
         work[r] = e - b;
+      }
+    }
+  }
+  if constexpr (SCAN) {
+    __shared__ uint64_t sh[kJSmallThreads / 32 + 1];
+    __syncthreads();  // this block wrote every work[r]
+    const uint64_t t = block_scan_write<kJSmallThreads>(work, (uint32_t)in.n, offs, sh);
+    if (threadIdx.x == 0) {
+      offs[in.n] = t;
+      if (ci.total) *ci.total = t;
+    }
+    if (pwork) {
+      const uint64_t pt = block_scan_write<kJSmallThreads>(pwork, (uint32_t)in.n, poffs, sh);
+      if (threadIdx.x == 0) {
+        poffs[in.n] = pt;
+        if (ci.ptotal) *ci.ptotal = pt;
       }
     }
   }
@@ -410,7 +444,16 @@ __global__ void __launch_bounds__(kJThreads) join_cj2_kernel(
   const int lane = threadIdx.x & 31;
   // (count-only rules never run in the device loop: the count instance
   // keeps the registers of the hot triangle level free of it)
-  if (MODE != kModeCount) total = dev_total(jd, total);
+  if (MODE == kModeTableCount && jd.d_total) {
+    // chunks past the true count are never taken: their counts are zero
+    const uint64_t ncap = (total + chunk - 1) / chunk;
+    total = dev_total(jd, total);
+    const uint64_t nt = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = (total + chunk - 1) / chunk + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < ncap; i += nt)
+      chunk_counts[i] = 0;
+  } else if (MODE != kModeCount) {
+    total = dev_total(jd, total);
+  }
   const uint32_t* vals0 = lv.src[0].prefix_slot < 0 ? lv.src[0].t.roots : lv.src[0].t.lo;
   const uint32_t* vals1 = lv.src[1].prefix_slot < 0 ? lv.src[1].t.roots : lv.src[1].t.lo;
   // a roots-list side with a dense directory answers membership in O(1)
@@ -788,11 +831,11 @@ __global__ void __launch_bounds__(kJThreads) join_cart2_kernel(
 
 size_t join_work_scratch_bytes(uint64_t rows) {
   rows = rows ? rows : 1;
-  // (+ the pivot rows' work, offsets and their scan)
+  // (+ the chunk queues; the pivot rows' work, offsets and their scan)
   return ((rows * 8 + 255) & ~size_t(255)) + ((rows + 1) * 8 + 255) + ((rows + 255) & ~size_t(255)) +
          2 * ((rows * 4 + 255) & ~size_t(255)) + ((rows * 8 + 255) & ~size_t(255)) +
          scan_scratch_bytes(rows) + 1024 + ((rows * 8 + 255) & ~size_t(255)) + ((rows + 1) * 8 + 511) +
-         scan_scratch_bytes(rows) + 512;
+         scan_scratch_bytes(rows) + 1024;
 }
 
 static int jgrid(uint64_t n, const Launch& L) {
@@ -1072,13 +1115,15 @@ __global__ void __launch_bounds__(kPvThreads, 1) join_pivot_count_kernel(
   }
 }
 
-JoinWork join_count(const Launch& L, const LevelSpec& lv, const Table& in, Scratch& s) {
+JoinWork join_count(const Launch& L, const LevelSpec& lv, const Table& in, Scratch& s, uint64_t* zero,
+                    uint64_t* total, uint64_t* ptotal) {
   JoinWork w;
   uint64_t* work = s.take<uint64_t>(in.n ? in.n : 1);
   w.offs = s.take<uint64_t>(in.n + 1);
   w.drv = s.take<uint8_t>(in.n ? in.n : 1);
   w.beg = s.take<uint32_t>(in.n ? in.n : 1);
   w.orange = s.take<uint2>(in.n ? in.n : 1);
+  w.queue = s.take<unsigned long long>(2);
   if (lv.kind == kColumnJoin && lv.nsrc == 2 && !lv.wide && (lv.src[0].t.bdir || lv.src[1].t.bdir))
     w.obm = s.take<uint32_t>(in.n ? in.n : 1);
   uint64_t* pwork = nullptr;
@@ -1086,14 +1131,24 @@ JoinWork join_count(const Launch& L, const LevelSpec& lv, const Table& in, Scrat
     pwork = s.take<uint64_t>(in.n);
     w.poffs = s.take<uint64_t>(in.n + 1);
   }
-  if (in.n) {
-    join_count_kernel<<<jgrid(in.n, L), kJThreads, 0, L.stream>>>(lv, in, work, w.drv,
-                                                                          w.beg, w.orange, w.obm, pwork);
+  CountInit ci{w.queue, zero, total, ptotal};
+  if (in.n && in.n <= kJSmallRows) {
+    join_count_kernel<true><<<1, kJSmallThreads, 0, L.stream>>>(lv, in, work, w.drv, w.beg, w.orange, w.obm, pwork,
+                                                                w.offs, w.poffs, ci);
     SRDL_CUDA(cudaGetLastError());
     count_launches(1);
+    return w;
   }
-  exclusive_scan_u64(L, work, in.n, w.offs, s);
-  if (pwork) exclusive_scan_u64(L, pwork, in.n, w.poffs, s);
+  if (in.n) {
+    join_count_kernel<false><<<jgrid(in.n, L), kJThreads, 0, L.stream>>>(lv, in, work, w.drv, w.beg, w.orange, w.obm,
+                                                                         pwork, nullptr, nullptr, ci);
+    SRDL_CUDA(cudaGetLastError());
+    count_launches(1);
+  } else if (zero) {
+    SRDL_CUDA(cudaMemsetAsync(zero, 0, 8, L.stream));
+  }
+  exclusive_scan_u64(L, work, in.n, w.offs, s, total);
+  if (pwork) exclusive_scan_u64(L, pwork, in.n, w.poffs, s, ptotal);
   return w;
 }
 
@@ -1173,8 +1228,7 @@ void join_expand(const Launch& L, const LevelSpec& lv, const Table& in, const Jo
     const uint64_t blocks = std::min<uint64_t>((uint64_t)L.num_sms * bpsm,
                                                (nchunks + kJThreads / 32 - 1) / (kJThreads / 32));
     const int gq = (int)std::max<uint64_t>(blocks, 1);
-    unsigned long long* q = s.take<unsigned long long>(2);
-    SRDL_CUDA(cudaMemsetAsync(q, 0, 2 * sizeof(unsigned long long), L.stream));
+    unsigned long long* q = w.queue;  // zeroed by the count launch
 #define SRDL_CJ2(MODE, Q, CC)                                                                     \
   (lv.seg ? join_cj2_kernel<MODE, true><<<gq, kJThreads, 0, L.stream>>>(                           \
                 lv, in, w.offs, w.drv, w.beg, w.orange, w.obm, total, chunk, Q, out, out_keys, cnt, \
@@ -1191,13 +1245,9 @@ void join_expand(const Launch& L, const LevelSpec& lv, const Table& in, const Jo
     } else {
       uint64_t* cc = s.take<uint64_t>(nchunks + 1);
       uint64_t* co = s.take<uint64_t>(nchunks + 1);
-      // with the count on the device, chunks past it are never taken: zero
-      // their counts so the scan over the capacity's chunks stays exact
-      if (jd.d_total) SRDL_CUDA(cudaMemsetAsync(cc, 0, (nchunks + 1) * 8, L.stream));
       SRDL_CJ2(kModeTableCount, q, cc);
       SRDL_CUDA(cudaGetLastError());
-      exclusive_scan_u64(L, cc, nchunks, co, s);
-      SRDL_CUDA(cudaMemcpyAsync(d_out_n, co + nchunks, 8, cudaMemcpyDeviceToDevice, L.stream));
+      exclusive_scan_u64(L, cc, nchunks, co, s, d_out_n);
       SRDL_CJ2(kModeTableWrite, q + 1, co);
       count_launches(2);
     }
@@ -1223,8 +1273,7 @@ void join_expand(const Launch& L, const LevelSpec& lv, const Table& in, const Jo
       uint64_t* wo = s.take<uint64_t>(warps + 1);
       SRDL_CART2(kModeTableCount, wc);
       SRDL_CUDA(cudaGetLastError());
-      exclusive_scan_u64(L, wc, warps, wo, s);
-      SRDL_CUDA(cudaMemcpyAsync(d_out_n, wo + warps, 8, cudaMemcpyDeviceToDevice, L.stream));
+      exclusive_scan_u64(L, wc, warps, wo, s, d_out_n);
       SRDL_CART2(kModeTableWrite, wo);
       count_launches(2);
     }
@@ -1248,8 +1297,7 @@ void join_expand(const Launch& L, const LevelSpec& lv, const Table& in, const Jo
     uint64_t* wo = s.take<uint64_t>(warps + 1);
     SRDL_EXP(kModeTableCount, wc);
     SRDL_CUDA(cudaGetLastError());
-    exclusive_scan_u64(L, wc, warps, wo, s);
-    SRDL_CUDA(cudaMemcpyAsync(d_out_n, wo + warps, 8, cudaMemcpyDeviceToDevice, L.stream));
+    exclusive_scan_u64(L, wc, warps, wo, s, d_out_n);
     SRDL_EXP(kModeTableWrite, wo);
     count_launches(2);
   }

@@ -109,15 +109,13 @@ void sort_dedup_dev(const Launch& L, const uint64_t* in, uint64_t cap, const uin
                     uint64_t* out, uint64_t out_cap, uint64_t* d_nout, unsigned int* d_overflow,
                     Scratch& s);
 
-// Trie view pieces for a sorted unique key array (with d_n: n is a capacity
-// and the count is on the device).
-size_t roots_scratch_bytes(uint64_t n);
-void build_lo(const Launch& L, const uint64_t* keys, uint64_t n, uint32_t* lo,
-              const uint64_t* d_n = nullptr);
-void build_dir(const Launch& L, const uint64_t* keys, uint64_t n, uint32_t* dir, uint32_t dir_n,
-               const uint64_t* d_n = nullptr);
-void build_roots(const Launch& L, const uint64_t* keys, uint64_t n, uint32_t* roots,
-                 uint64_t* d_nroots, Scratch& s, const uint64_t* d_n = nullptr);
+// Trie view of a sorted unique key array (with d_n: n is a capacity
+// and the count is on the device): the child column lo, the distinct first
+// values roots (their count to *d_nroots) and, with dir_n > 0, the dense
+// directory.
+size_t trie_scratch_bytes(uint64_t n);
+void build_trie(const Launch& L, const uint64_t* keys, uint64_t n, uint32_t* lo, uint32_t* roots,
+                uint64_t* d_nroots, uint32_t* dir, uint32_t dir_n, Scratch& s, const uint64_t* d_n = nullptr);
 
 // Hash tables for the child lists longer than `min_len` of a dense-directory
 // trie.  Plan: sizes[v] = slots for value v (0 = no table), offs = exclusive
@@ -177,10 +175,11 @@ void split3(const Launch& L, const uint64_t* keys, uint64_t n, int bits, int hal
 // Swap the two 32-bit halves of every key (index permutation (1,0) <-> (0,1)).
 void swap_halves(const Launch& L, const uint64_t* in, uint64_t n, uint64_t* out);
 
-// Exclusive scan of n uint64 values; out has n+1 entries (out[n] = total).
+// Exclusive scan of n uint64 values; out has n+1 entries (out[n] = total, also
+// written to *total when given).
 size_t scan_scratch_bytes(uint64_t n);
 void exclusive_scan_u64(const Launch& L, const uint64_t* in, uint64_t n, uint64_t* out,
-                        Scratch& s);
+                        Scratch& s, uint64_t* total = nullptr);
 
 // ---------------------------------------------------------------- join
 constexpr int kMaxSlots = 8;
@@ -278,8 +277,13 @@ struct JoinWork {
   uint2* orange = nullptr;   // two-source column join: the other list [x, y) per row
   uint32_t* obm = nullptr;   // two-source column join: bitmap slot of the other list, or kNoBitmap
   uint64_t* poffs = nullptr; // pivot rows (lv.pivot_src): prefix sums of their candidates, rows + 1
+  unsigned long long* queue = nullptr;  // two zeroed words: chunk queues of the two-source column join
 };
-JoinWork join_count(const Launch& L, const LevelSpec& lv, const Table& in, Scratch& s);
+// zero: a word the pass sets to 0 (may be null); total / ptotal: where the
+// totals of offs / poffs go besides (device or page-locked host memory; may
+// be null).
+JoinWork join_count(const Launch& L, const LevelSpec& lv, const Table& in, Scratch& s, uint64_t* zero = nullptr,
+                    uint64_t* total = nullptr, uint64_t* ptotal = nullptr);
 
 // Shared memory the pivot kernel needs for a bitmap of the values that a dense
 // directory of dir_n entries covers; levels that need more than kPivotSmemMax
@@ -293,7 +297,8 @@ constexpr size_t kPivotSmemMax = 200 * 1024;
 // with lv.seg set this shard's segments of them, total = seg_owned(...));
 // surviving bindings are appended to `out_table` (emit table, in input
 // order: the table stays sorted), to `out_keys` (emit keys, any order) or
-// counted (emit count) via *d_out_n, which the caller zeroes.  Output
+// counted (emit count) via *d_out_n, which the caller zeroes for emit keys and
+// emit count (emit table sets it).  Output
 // capacity = total.  The scratch for a level of `total` candidates comes
 // from join_expand_scratch_bytes(L, total).
 size_t join_expand_scratch_bytes(const Launch& L, uint64_t total);

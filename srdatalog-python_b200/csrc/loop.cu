@@ -262,7 +262,7 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
       }
       lr.newk = DevBuf(lr.cap_new * 8, L_.stream);
       lr.sort_scr = DevBuf(sort_dev_scratch_bytes(lr.cap_new, lr.cap_full, bits_), L_.stream);
-      lr.trie_scr = DevBuf(roots_scratch_bytes(lr.cap_delta) + 1024, L_.stream);
+      lr.trie_scr = DevBuf(trie_scratch_bytes(lr.cap_delta) + 1024, L_.stream);
       for (int q = 0; q < 2; q++) {
         lr.full[q] = DevBuf(lr.cap_full * 8, L_.stream);
         lr.delta[q] = DevBuf(lr.cap_delta * 8, L_.stream);
@@ -327,11 +327,8 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
       SRDL_CUDA(cudaMemcpyAsync(lr.delta[0].as<void>(), dit->second.keys.as<void>(), dn * 8,
                                 cudaMemcpyDeviceToDevice, L_.stream));
     Scratch ts{lr.trie_scr.as<char>(), lr.trie_scr.bytes(), 0};
-    build_lo(L_, lr.delta[0].as<uint64_t>(), lr.cap_delta, lr.lo[0].as<uint32_t>(), &c->n_delta[0]);
-    build_roots(L_, lr.delta[0].as<uint64_t>(), lr.cap_delta, lr.roots[0].as<uint32_t>(), &c->n_roots[0], ts,
-                &c->n_delta[0]);
-    build_dir(L_, lr.delta[0].as<uint64_t>(), lr.cap_delta, lr.dir[0].as<uint32_t>(), X.dir_n,
-              &c->n_delta[0]);
+    build_trie(L_, lr.delta[0].as<uint64_t>(), lr.cap_delta, lr.lo[0].as<uint32_t>(), lr.roots[0].as<uint32_t>(),
+               &c->n_roots[0], lr.dir[0].as<uint32_t>(), X.dir_n, ts, &c->n_delta[0]);
   }
   {
     // (a fixpoint always converges; the cap bounds one graph launch should
@@ -394,7 +391,9 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
   auto body = [&](int p, cudaGraphConditionalHandle hw, cudaGraphConditionalHandle hi, int set_if) {
     LoopCounts* cnt = X.cnt_d();
     unsigned int* ovf = &X.ctl_d()->overflow;
-    for (size_t i = 0; i < X.rels.size(); i++) SRDL_CUDA(cudaMemsetAsync(&cnt[i].n_new, 0, 8, L_.stream));
+    std::vector<char> zeroed(X.rels.size(), 0);  // n_new of the relations a rule has begun to fill
+    for (size_t i = 0; i < X.rels.size(); i++)
+      if (!X.rels[i].producers) SRDL_CUDA(cudaMemsetAsync(&cnt[i].n_new, 0, 8, L_.stream));
     const std::map<std::string, TrieView> dv = delta_views(p);
     for (size_t k = 0; k < execs.size(); k++) {
       const Op& op = *execs[k];
@@ -411,7 +410,9 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
         LoopLevel& ll = lvls[li];
         const bool last = li + 1 == pp.levels.size();
         Scratch s{ll.wscr.as<char>(), ll.wscr.bytes(), 0};
-        JoinWork w = join_count(L_, lv, cur, s);
+        // a relation's first rule zeroes its count of new keys
+        JoinWork w = join_count(L_, lv, cur, s, li == 0 && !zeroed[ri] ? &cnt[ri].n_new : nullptr);
+        if (li == 0) zeroed[ri] = 1;
         Scratch xs{ll.xscr.as<char>(), ll.xscr.bytes(), 0};
         JoinDev jd;
         jd.d_total = w.offs + cur.n;
@@ -432,7 +433,6 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
             SRDL_REQUIRE(ll.cols[c].bytes() > 0, kErrState, "device loop: table column missing");
             next.col[c] = ll.cols[c].as<uint32_t>();
           }
-          SRDL_CUDA(cudaMemsetAsync(ll.count.as<void>(), 0, 8, L_.stream));
           jd.out_cap = ll.cap_total;
           join_expand(L_, lv, cur, w, ll.cap_total, &next, nullptr, ll.count.as<uint64_t>(), xs, &jd);
           next.n = ll.cap_total;
@@ -453,11 +453,9 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
                          lr.delta[1 - p].as<uint64_t>(), lr.cap_delta, &c->n_delta[1 - p],
                          lr.full[1 - p].as<uint64_t>(), lr.cap_full, &c->n_full[1 - p], ovf);
       Scratch ts{lr.trie_scr.as<char>(), lr.trie_scr.bytes(), 0};
-      build_lo(L_, lr.delta[1 - p].as<uint64_t>(), lr.cap_delta, lr.lo[1 - p].as<uint32_t>(), &c->n_delta[1 - p]);
-      build_roots(L_, lr.delta[1 - p].as<uint64_t>(), lr.cap_delta, lr.roots[1 - p].as<uint32_t>(),
-                  &c->n_roots[1 - p], ts, &c->n_delta[1 - p]);
-      build_dir(L_, lr.delta[1 - p].as<uint64_t>(), lr.cap_delta, lr.dir[1 - p].as<uint32_t>(), X.dir_n,
-                &c->n_delta[1 - p]);
+      build_trie(L_, lr.delta[1 - p].as<uint64_t>(), lr.cap_delta, lr.lo[1 - p].as<uint32_t>(),
+                 lr.roots[1 - p].as<uint32_t>(), &c->n_roots[1 - p], lr.dir[1 - p].as<uint32_t>(), X.dir_n, ts,
+                 &c->n_delta[1 - p]);
       // batched runs: the instances with a delta row in this iteration
       // (its number is it0 + 1 + the bodies started before it)
       if (loop_marks_)

@@ -887,18 +887,17 @@ void Database::ensure_trie(Relation& r, Index& ix, int64_t hi_max) {
   size_t pid = prof_begin("trie_build");
   ix.lo = DevBuf(std::max<uint64_t>(n, 1) * 4, L_.stream);
   ix.roots = DevBuf(std::max<uint64_t>(n, 1) * 4, L_.stream);
-  build_lo(L_, ix.keys.as<uint64_t>(), n, ix.lo.as<uint32_t>());
-  DevBuf scratch(roots_scratch_bytes(n) + 1024, L_.stream);
+  DevBuf scratch(trie_scratch_bytes(n) + 1024, L_.stream);
   Scratch s{scratch.as<char>(), scratch.bytes(), 0};
   // the root count stays on the device: kernels read it, the host never waits for it
   ix.nroots_d = DevBuf(8, L_.stream);
-  build_roots(L_, ix.keys.as<uint64_t>(), n, ix.roots.as<uint32_t>(), ix.nroots_d.as<uint64_t>(), s);
   ix.dir_n = 0;
   if (hmax + 2 <= kDenseDirMax) {
     ix.dir_n = (uint32_t)(hmax + 2);
     ix.dir = DevBuf((size_t)ix.dir_n * 4, L_.stream);
-    build_dir(L_, ix.keys.as<uint64_t>(), n, ix.dir.as<uint32_t>(), ix.dir_n);
   }
+  build_trie(L_, ix.keys.as<uint64_t>(), n, ix.lo.as<uint32_t>(), ix.roots.as<uint32_t>(),
+             ix.nroots_d.as<uint64_t>(), ix.dir_n ? ix.dir.as<uint32_t>() : nullptr, ix.dir_n, s);
   prof_end(pid, 8.0 * n + 4.0 * n + 8.0 * n + 4.0 * ix.dir_n, (double)n);
   ix.trie = true;
 }

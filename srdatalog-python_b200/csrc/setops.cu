@@ -185,19 +185,41 @@ void set_difference(const Launch& L, const uint64_t* a, uint64_t na, const uint6
   compact_diff(L, sel, na, d_nout, s);
 }
 
-__global__ void lo_kernel(const uint64_t* __restrict__ keys, uint64_t n, uint32_t* __restrict__ lo,
-                          const uint64_t* d_n) {
+// First pass of a trie view: the child column, the flag words and per-block
+// counts of the first-column values (blocks below nb, `chunk` keys each), and
+// the dense directory (all blocks).  Each key is read once; its predecessor's
+// first column comes from the neighbouring lane.
+__global__ void __launch_bounds__(kCpThreads) trie_kernel(const uint64_t* __restrict__ keys, uint64_t n, int nb,
+                                                          uint64_t chunk, uint32_t* __restrict__ lo,
+                                                          uint32_t* __restrict__ flags,
+                                                          uint32_t* __restrict__ blk_counts,
+                                                          uint32_t* __restrict__ dir, uint32_t dir_n,
+                                                          const uint64_t* d_n) {
+  __shared__ uint32_t sh[kCpThreads / 32 + 1];
   n = dev_size(n, d_n);
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-       i += (uint64_t)gridDim.x * blockDim.x)
-    lo[i] = (uint32_t)keys[i];
-}
-
-__global__ void dir_kernel(const uint64_t* __restrict__ keys, uint64_t n, uint32_t* __restrict__ dir,
-                           uint32_t dir_n, const uint64_t* d_n) {
-  n = dev_size(n, d_n);
-  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < dir_n;
-       v += (uint64_t)gridDim.x * blockDim.x)
+  if ((int)blockIdx.x < nb) {
+    if (d_n) chunk = cp_even_chunk(n, nb);
+    const uint64_t begin = (uint64_t)blockIdx.x * chunk;
+    const uint64_t end = begin + chunk < n ? begin + chunk : n;
+    const int lane = threadIdx.x & 31;
+    uint32_t cnt = 0;
+    for (uint64_t w0 = begin + (threadIdx.x & ~31u); w0 < end; w0 += kCpThreads) {
+      const uint64_t i = w0 + lane;
+      const uint64_t k = i < end ? __ldg(keys + i) : 0;
+      const uint32_t hi = (uint32_t)(k >> 32);
+      uint32_t before = __shfl_up_sync(kAllLanes, hi, 1);
+      if (lane == 0 && w0 > 0) before = (uint32_t)(__ldg(keys + w0 - 1) >> 32);
+      const bool f = i < end && (i == 0 || hi != before);
+      if (i < end) lo[i] = (uint32_t)k;
+      const uint32_t m = __ballot_sync(kAllLanes, f);
+      if (lane == 0) flags[w0 / 32] = m;
+      cnt += f;
+    }
+    uint32_t tot;
+    block_excl_scan(cnt, sh, &tot);
+    if (threadIdx.x == 0) blk_counts[blockIdx.x] = tot;
+  }
+  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < dir_n; v += (uint64_t)gridDim.x * blockDim.x)
     dir[v] = (uint32_t)lower_bound_u64(keys, 0, n, v << 32);
 }
 
@@ -216,27 +238,25 @@ static int grid_for(uint64_t n, int sms) {
   return g ? (int)g : 1;
 }
 
-void build_lo(const Launch& L, const uint64_t* keys, uint64_t n, uint32_t* lo, const uint64_t* d_n) {
-  if (!n) return;
-  lo_kernel<<<grid_for(n, L.num_sms), 256, 0, L.stream>>>(keys, n, lo, d_n);
-  SRDL_CUDA(cudaGetLastError());
+size_t trie_scratch_bytes(uint64_t n) { return cp_scratch_bytes(n); }
+
+void build_trie(const Launch& L, const uint64_t* keys, uint64_t n, uint32_t* lo, uint32_t* roots,
+                uint64_t* d_nroots, uint32_t* dir, uint32_t dir_n, Scratch& s, const uint64_t* d_n) {
+  const uint64_t chunk = cp_chunk(n, L.num_sms);
+  const int nb = n ? cp_blocks(n, chunk) : 0;
+  if (!n) SRDL_CUDA(cudaMemsetAsync(d_nroots, 0, sizeof(uint64_t), L.stream));
+  const int grid = std::max(nb, dir_n ? grid_for(dir_n, L.num_sms) : 0);
+  if (!grid) return;
+  uint32_t* flags = s.take<uint32_t>(cp_words(n));
+  uint32_t* counts = s.take<uint32_t>(nb ? nb : 1);
+  trie_kernel<<<grid, kCpThreads, 0, L.stream>>>(keys, n, nb, chunk, lo, flags, counts, dir, dir_n, d_n);
   count_launches(1);
-}
-
-void build_dir(const Launch& L, const uint64_t* keys, uint64_t n, uint32_t* dir, uint32_t dir_n,
-               const uint64_t* d_n) {
-  if (!dir_n) return;
-  dir_kernel<<<grid_for(dir_n, L.num_sms), 256, 0, L.stream>>>(keys, n, dir, dir_n, d_n);
+  if (nb) {
+    cp_write_kernel<RootSel><<<nb, kCpThreads, 0, L.stream>>>(RootSel{keys, roots}, n, d_n ? 0 : chunk, flags, counts,
+                                                              d_nroots, d_n);
+    count_launches(1);
+  }
   SRDL_CUDA(cudaGetLastError());
-  count_launches(1);
-}
-
-size_t roots_scratch_bytes(uint64_t n) { return cp_scratch_bytes(n); }
-
-void build_roots(const Launch& L, const uint64_t* keys, uint64_t n, uint32_t* roots,
-                 uint64_t* d_nroots, Scratch& s, const uint64_t* d_n) {
-  RootSel sel{keys, roots};
-  compact(L, sel, n, d_nroots, s, d_n);
 }
 
 void swap_halves(const Launch& L, const uint64_t* in, uint64_t n, uint64_t* out) {
@@ -521,30 +541,37 @@ __global__ void __launch_bounds__(kScThreads) scan_sum_kernel(const uint64_t* __
   if (threadIdx.x == 0) bsum[blockIdx.x] = tot;
 }
 
-__global__ void scan_blocks_kernel(uint64_t* bsum, int nb) {
-  __shared__ uint64_t sh[1024 / 32 + 1];
-  const int per = (nb + blockDim.x - 1) / blockDim.x;
-  const int s = threadIdx.x * per, e = min(nb, s + per);
-  uint64_t sum = 0;
-  for (int i = s; i < e; i++) sum += bsum[i];
-  uint64_t tot;
-  uint64_t run = block_excl_scan(sum, sh, &tot);
-  for (int i = s; i < e; i++) {
-    uint64_t v = bsum[i];
-    bsum[i] = run;
-    run += v;
+// One block, one launch: kScSmall values at most.
+constexpr int kScSmallThreads = 1024;
+constexpr uint64_t kScSmall = 16384;
+
+__global__ void __launch_bounds__(kScSmallThreads) scan_small_kernel(const uint64_t* __restrict__ in, uint32_t n,
+                                                                     uint64_t* __restrict__ out,
+                                                                     uint64_t* __restrict__ total) {
+  __shared__ uint64_t sh[kScSmallThreads / 32 + 1];
+  const uint64_t tot = block_scan_write<kScSmallThreads>(in, n, out, sh);
+  if (threadIdx.x == 0) {
+    out[n] = tot;
+    if (total) *total = tot;
   }
-  if (threadIdx.x == 0) bsum[nb] = tot;
 }
 
+// Every block adds up the sums of the blocks before it (at most 8 per SM)
+// instead of waiting for a launch of its own to scan them.
 __global__ void __launch_bounds__(kScThreads) scan_write_kernel(const uint64_t* __restrict__ in,
                                                                 uint64_t n, uint64_t chunk,
-                                                                const uint64_t* __restrict__ boff,
-                                                                uint64_t* __restrict__ out) {
+                                                                const uint64_t* __restrict__ bsum,
+                                                                uint64_t* __restrict__ out,
+                                                                uint64_t* __restrict__ total) {
   __shared__ uint64_t sh[kScThreads / 32 + 1];
   const uint64_t begin = (uint64_t)blockIdx.x * chunk;
   const uint64_t end = begin + chunk < n ? begin + chunk : n;
-  uint64_t base = boff[blockIdx.x];
+  uint64_t base = block_prefix(bsum, blockIdx.x, sh);
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+    const uint64_t t = base + bsum[blockIdx.x];
+    out[n] = t;
+    if (total) *total = t;
+  }
   for (uint64_t tile = begin; tile < end; tile += kScTile) {
     const uint64_t i0 = tile + (uint64_t)threadIdx.x * kScItems;
     uint64_t v[kScItems];
@@ -563,15 +590,16 @@ __global__ void __launch_bounds__(kScThreads) scan_write_kernel(const uint64_t* 
     }
     base += tot;
   }
-  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = boff[gridDim.x];
 }
 
 size_t scan_scratch_bytes(uint64_t) { return (size_t)(256 * 8 + 2) * 8 + 512; }
 
 void exclusive_scan_u64(const Launch& L, const uint64_t* in, uint64_t n, uint64_t* out,
-                        Scratch& s) {
-  if (n == 0) {
-    SRDL_CUDA(cudaMemsetAsync(out, 0, sizeof(uint64_t), L.stream));
+                        Scratch& s, uint64_t* total) {
+  if (n <= kScSmall) {
+    scan_small_kernel<<<1, kScSmallThreads, 0, L.stream>>>(in, (uint32_t)n, out, total);
+    SRDL_CUDA(cudaGetLastError());
+    count_launches(1);
     return;
   }
   const uint64_t tiles = (n + kScTile - 1) / kScTile;
@@ -581,10 +609,9 @@ void exclusive_scan_u64(const Launch& L, const uint64_t* in, uint64_t n, uint64_
   const int nb = (int)((n + chunk - 1) / chunk);
   uint64_t* bsum = s.take<uint64_t>(nb + 1);
   scan_sum_kernel<<<nb, kScThreads, 0, L.stream>>>(in, n, chunk, bsum);
-  scan_blocks_kernel<<<1, 1024, 0, L.stream>>>(bsum, nb);
-  scan_write_kernel<<<nb, kScThreads, 0, L.stream>>>(in, n, chunk, bsum, out);
+  scan_write_kernel<<<nb, kScThreads, 0, L.stream>>>(in, n, chunk, bsum, out, total);
   SRDL_CUDA(cudaGetLastError());
-  count_launches(3);
+  count_launches(2);
 }
 
 }  // namespace srdl

@@ -36,25 +36,6 @@ int value_bits(uint32_t max_value) {
   return b ? b : 1;
 }
 
-__global__ void cp_scan_kernel(const uint32_t* blk_counts, int nb, uint64_t* offs,
-                               uint64_t* d_total) {
-  __shared__ uint64_t sh[1024 / 32 + 1];
-  const int per = (nb + blockDim.x - 1) / blockDim.x;
-  const int s = threadIdx.x * per, e = min(nb, s + per);
-  uint64_t sum = 0;
-  for (int i = s; i < e; i++) sum += blk_counts[i];
-  uint64_t tot;
-  uint64_t run = block_excl_scan(sum, sh, &tot);
-  for (int i = s; i < e; i++) {
-    offs[i] = run;
-    run += blk_counts[i];
-  }
-  if (threadIdx.x == 0) {
-    offs[nb] = tot;
-    *d_total = tot;
-  }
-}
-
 template <typename K>
 __global__ void rs_pack(const uint64_t* __restrict__ in, uint64_t n, int bits, bool swap,
                         K* __restrict__ out, const uint64_t* d_n) {

@@ -8,9 +8,32 @@ import pytest
 from conftest import load_plan
 from srdatalog_b200 import native
 from srdatalog_b200 import workloads as W
+from test_gpu_primitives import gpu_merge, keys_with_bits
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip('torch')
+
+
+@pytest.mark.parametrize('na,nb', [(1, 2047), (2048, 0), (2048, 2048), (2049, 4095), (1, 2_000_000),
+                                   (2048 * 148 * 6, 5)])
+@pytest.mark.parametrize('apart', [False, True])
+def test_merge_tile_edges(na, nb, apart):
+  rng = np.random.default_rng(na + 7 * nb)
+  u = np.unique(keys_with_bits(rng, na + nb + 10, 28))[:na + nb]
+  if not apart:
+    rng.shuffle(u)
+  a, b = np.sort(u[:na]), np.sort(u[na:])
+  assert np.array_equal(gpu_merge(a, b), oracle.merge(a, b))
+
+
+@pytest.mark.parametrize('m', [4095, 4096, 4097, 16_384, 16_385, 120_000])
+def test_count_scan_edges(m):
+  '''Tables on both sides of the one-block count and scan.'''
+  e = W.rmat_edges(13, 2 * m, seed=m)[:m]
+  with native.Database(load_plan('triangle')) as db:
+    db.load_rows('KnowsInput', e)
+    db.run()
+    assert db.count('TriangleJoin') == oracle.triangle_count(e)
 
 
 @pytest.mark.parametrize('pivot_min', [1, 3, 64, 1 << 20])
