@@ -30,6 +30,13 @@ constexpr int kCpWarps = kCpThreads / 32;
 constexpr int kCpItems = 8;
 constexpr int kCpTile = kCpThreads * kCpItems;
 
+// Largest FULL, in multiples of the keys, that a set difference streams (its
+// merge path); past it every key is searched in FULL (its probe path).
+// Measured, merge / probe: 1M keys against 4M 69 / 55 us and against 8M 85 / 55
+// us, 10M against 30M 267 / 271 us; but 10M against 15M 193 / 247 us and 50M
+// against 30M 549 / 957 us.
+constexpr uint64_t kDmMaxFullRatio = 2;
+
 // Grid shape for n elements: every block owns `chunk` elements (a multiple
 // of the tile), at most 8 blocks per SM, no empty blocks.
 inline uint64_t cp_chunk(uint64_t n, int sms) {
@@ -50,15 +57,13 @@ __device__ __forceinline__ uint64_t cp_even_chunk(uint64_t n, uint64_t nb) {
 }
 inline uint64_t cp_words(uint64_t n) { return (n + 31) / 32; }
 inline size_t cp_scratch_bytes(uint64_t n) {
-  // flag words + per-block counts and offsets (blocks <= 8 per SM; 256 SMs
-  // bound) + the FULL and HEAD positions of every tile boundary (set
-  // difference), each piece padded to 256 bytes, plus alignment slack for the
-  // region itself
-  // (+ the merge-path cuts: FULL at most 16 times the keys on that path)
-  const uint64_t tiles = (n + kCpTile - 1) / kCpTile + 1;
-  const uint64_t mtiles = (17 * n + kCpTile - 1) / kCpTile + 2;
-  return ((cp_words(n) * 4 + 255) & ~uint64_t(255)) + (size_t)(256 * 8 + 1) * 12 + 3 * 256 +
-         2 * ((tiles * 8 + 255) & ~uint64_t(255)) + 2 * ((mtiles * 8 + 255) & ~uint64_t(255)) + 256;
+  // flag words + per-block counts (blocks <= 8 per SM; 256 SMs bound), and for
+  // the set difference the merge-path cuts and HEAD positions of every tile
+  // boundary (FULL at most kDmMaxFullRatio times the keys there), each piece
+  // padded to 256 bytes, plus alignment slack for the region itself
+  const uint64_t mtiles = ((kDmMaxFullRatio + 1) * n + kCpTile - 1) / kCpTile + 2;
+  return ((cp_words(n) * 4 + 255) & ~uint64_t(255)) + (size_t)(256 * 8 + 1) * 4 + 3 * 256 +
+         2 * ((mtiles * 8 + 255) & ~uint64_t(255)) + 256;
 }
 
 // With d_n (device loop), n is a capacity and the count is *d_n; chunk 0
@@ -182,31 +187,9 @@ struct DedupDiffSel {
     const uint64_t m = (1ull << bits) - 1;
     return (((uint64_t)c >> bits) << 32) | ((uint64_t)c & m);
   }
-  __device__ void block_setup(uint64_t begin, uint64_t end) {
-    __shared__ uint64_t range[2];
-    if (full && n_full) {
-      if (threadIdx.x == 0 && begin < end) {
-        range[0] = lower_bound_u64(full, 0, n_full, expand(a[begin]));
-        uint64_t last = expand(a[end - 1]);
-        uint64_t hi = lower_bound_u64(full, range[0], n_full, last);
-        range[1] = (hi < n_full && full[hi] == last) ? hi + 1 : hi;
-      }
-      __syncthreads();
-      lo_ = range[0];
-      hi_ = range[1];
-    }
-  }
-  uint64_t lo_ = 0, hi_ = 0;
-  __device__ bool select(uint64_t i) const {
-    K c = a[i];
-    if (dedup && i > 0 && a[i - 1] == c) return false;
-    if (full && hi_ > lo_) {
-      uint64_t k = expand(c);
-      uint64_t p = lower_bound_u64(full, lo_, hi_, k);
-      if (p < hi_ && full[p] == k) return false;
-    }
-    return true;
-  }
+  __device__ void block_setup(uint64_t, uint64_t) {}
+  // (without FULL and HEAD: compact_diff takes the paths below otherwise)
+  __device__ bool select(uint64_t i) const { return !(dedup && i > 0 && a[i - 1] == a[i]); }
   using value_type = uint64_t;
   __device__ uint64_t value(uint64_t i) const { return expand(a[i]); }
   __device__ void store(uint64_t pos, uint64_t v) const {
@@ -215,59 +198,51 @@ struct DedupDiffSel {
   }
 };
 
-// FULL position of every tile boundary: fpos[t] = lower_bound(FULL, first key
-// of tile t) for t < tiles, fpos[tiles] = n_full.  One warp per boundary
-// (32-ary search), all boundaries in parallel.  Tile t's keys can only match
-// FULL[fpos[t], fpos[t+1] + 1): its last key is <= the next tile's first.
-// hpos (when a HEAD is given) holds the same positions in HEAD.
+// Device loop (d_n set): the merge path and the probe path are both in the
+// graph and each kernel runs only when the counts on the device select its
+// path.  The merge path streams all of FULL; the probe path costs a binary
+// search in FULL per key and nothing else.
+enum DiffPath : int { kPathAny = 0, kPathMerge = 1, kPathProbe = 2 };
+
 template <typename K>
-__global__ void dd_bounds_kernel(DedupDiffSel<K> sel, uint64_t n, uint64_t tiles,
-                                 uint64_t* __restrict__ fpos, uint64_t* __restrict__ hpos,
-                                 const uint64_t* d_n, int path) {
-  sel.n_full = dev_size(sel.n_full, sel.d_n_full);
-  n = dev_size(n, d_n);
-  if (!diff_path_runs(path, sel, n)) return;
-  const uint64_t real = (n + kCpTile - 1) / kCpTile;  // tiles holding keys
-  // one warp per boundary; warps walk the boundaries when the grid is capped
-  const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) / 32;
-  for (uint64_t t = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / 32; t <= tiles; t += warps) {
-    uint64_t p = sel.n_full, q = sel.n_head;
-    if (t < real) {
-      const uint64_t first = sel.expand(sel.a[t * kCpTile]);
-      p = warp_partition_point(0, sel.n_full, [&](uint64_t i) { return sel.full[i] < first; });
-      if (hpos)
-        q = warp_partition_point(0, sel.n_head, [&](uint64_t i) { return sel.head[i] < first; });
-    }
-    if ((threadIdx.x & 31) == 0) {
-      fpos[t] = p;
-      if (hpos) hpos[t] = q;
-    }
-    if (d_n && t > real) break;  // past the true tiles every entry is n_full
-  }
+__device__ __forceinline__ bool diff_path_runs(int path, const DedupDiffSel<K>& sel, uint64_t n) {
+  if (path == kPathAny) return true;
+  const bool merge = sel.n_full <= kDmMaxFullRatio * n;
+  return (path == kPathMerge) == merge;
 }
 
-// Flag pass of DedupDiffSel with FULL: the block walks its chunk one tile at
-// a time and stages the tile's keys and, when it fits, the tile's slice of
-// FULL in shared memory.  Thread t owns the tile's keys [8t, 8t + 8): it
-// binary-searches the slice for its first key only and walks forward from
-// there for the other seven (both runs are sorted), so a key costs about one
-// comparison instead of a dozen.  The eight flag bits of four neighbouring
-// threads form one 32-key flag word.  Slices that do not fit are searched in
-// global memory, each key galloping forward from the previous key's
-// position; the HEAD segment is probed by binary search within the tile's
-// range.
-constexpr int kDdStage = 4000;  // FULL keys staged per tile (31.25 KB: with 64-bit tile keys under 48 KB)
+// lower_bound of kDdKeys keys of one lane in a[0..n) (n > 0): the halvings are
+// the same for every key, so the lane keeps kDdKeys loads in flight.
+constexpr int kDdKeys = 8;
+__device__ __forceinline__ void dd_lower_bounds(const uint64_t* __restrict__ a, uint64_t n,
+                                                const uint64_t (&k)[kDdKeys], bool (&found)[kDdKeys]) {
+  uint64_t p[kDdKeys];
+#pragma unroll
+  for (int q = 0; q < kDdKeys; q++) p[q] = 0;
+  while (n > 1) {
+    const uint64_t half = n >> 1;
+#pragma unroll
+    for (int q = 0; q < kDdKeys; q++)
+      if (__ldg(a + p[q] + half) <= k[q]) p[q] += half;
+    n -= half;
+  }
+#pragma unroll
+  for (int q = 0; q < kDdKeys; q++) found[q] = __ldg(a + p[q]) == k[q];
+}
 
+// Probe path: flag words and per-block counts by one binary search per key in
+// FULL (and HEAD).  A warp takes eight rounds of 32 consecutive keys at a
+// time, one search per round and lane, all eight interleaved: a late
+// iteration's few keys would otherwise pay eight searches of about 23
+// dependent loads one after another.  Neighbouring lanes' keys are
+// neighbours, so the last steps of a round's searches share lines.  30k keys
+// against 8M: 50 us for the whole set difference, 103 us with eight searches
+// one after another per thread.
 template <typename K>
-__global__ void __launch_bounds__(kCpThreads) dd_flag_kernel(DedupDiffSel<K> sel, uint64_t n,
-                                                             uint64_t chunk,
-                                                             const uint64_t* __restrict__ fpos,
-                                                             const uint64_t* __restrict__ hpos,
-                                                             uint32_t* flags,
-                                                             uint32_t* blk_counts,
-                                                             const uint64_t* d_n, int path) {
-  __shared__ uint64_t stage[kDdStage];
-  __shared__ K skey[kCpTile + 1];  // skey[j + 1] = tile key j, skey[0] = the key before the tile
+__global__ void __launch_bounds__(kCpThreads) dd_probe_kernel(DedupDiffSel<K> sel, uint64_t n, uint64_t chunk,
+                                                              uint32_t* __restrict__ flags,
+                                                              uint32_t* __restrict__ blk_counts,
+                                                              const uint64_t* d_n, int path) {
   __shared__ uint32_t sh[kCpThreads / 32 + 1];
   sel.n_full = dev_size(sel.n_full, sel.d_n_full);
   n = dev_size(n, d_n);
@@ -275,105 +250,38 @@ __global__ void __launch_bounds__(kCpThreads) dd_flag_kernel(DedupDiffSel<K> sel
   chunk = dev_chunk(chunk, n, kCpTile);
   const uint64_t begin = (uint64_t)blockIdx.x * chunk;
   const uint64_t end = begin + chunk < n ? begin + chunk : n;
-  const int lane = threadIdx.x & 31;
-  const uint32_t j0 = threadIdx.x * kCpItems;
-  uint32_t cnt = 0;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  uint32_t cnt = 0;  // (lane 0: the warp's)
   for (uint64_t tile = begin; tile < end; tile += kCpTile) {
-    const uint32_t tn = (uint32_t)(end - tile < kCpTile ? end - tile : kCpTile);
-    const uint64_t t = tile / kCpTile;
-    const uint64_t f0 = fpos[t];
-    uint64_t f1 = fpos[t + 1] + 1;
-    f1 = f1 < sel.n_full ? f1 : sel.n_full;
-    const uint32_t len = (uint32_t)(f1 > f0 ? (f1 - f0 < 0xffffffffull ? f1 - f0 : 0xffffffffull) : 0);
-    const bool staged = len <= (uint32_t)kDdStage;
-    uint64_t h0 = 0, h1 = 0;
-    if (hpos) {
-      h0 = hpos[t];
-      h1 = hpos[t + 1] + 1;
-      h1 = h1 < sel.n_head ? h1 : sel.n_head;
+    const uint64_t w0 = tile + (uint64_t)wid * (kDdKeys * 32);
+    uint64_t k[kDdKeys];
+    bool keep[kDdKeys], hit[kDdKeys];
+#pragma unroll
+    for (int q = 0; q < kDdKeys; q++) {
+      const uint64_t i = w0 + q * 32 + lane;
+      const K c = i < end ? sel.a[i] : K(0);
+      keep[q] = i < end && !(sel.dedup && i > 0 && sel.a[i - 1] == c);
+      k[q] = sel.expand(c);
     }
-    // Staging: every thread issues all of its loads before its first shared
-    // store, so a tile costs one or two memory round trips, not one per load.
-    {
-      K kr[kCpItems];
+    if (sel.n_full) {
+      dd_lower_bounds(sel.full, sel.n_full, k, hit);
 #pragma unroll
-      for (int q = 0; q < kCpItems; q++) {
-        const uint32_t j = threadIdx.x + q * kCpThreads;
-        kr[q] = j < tn ? sel.a[tile + j] : K(0);
-      }
-      const K prev = (threadIdx.x == 0 && tile > 0) ? sel.a[tile - 1] : K(0);
-      if (staged) {
-        for (uint32_t b0 = 0; b0 < len; b0 += kCpThreads * kCpItems) {
-          uint64_t fr[kCpItems];
-#pragma unroll
-          for (int q = 0; q < kCpItems; q++) {
-            const uint32_t j = b0 + threadIdx.x + q * kCpThreads;
-            fr[q] = j < len ? sel.full[f0 + j] : 0;
-          }
-#pragma unroll
-          for (int q = 0; q < kCpItems; q++) {
-            const uint32_t j = b0 + threadIdx.x + q * kCpThreads;
-            if (j < len) stage[j] = fr[q];
-          }
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < kCpItems; q++) {
-        const uint32_t j = threadIdx.x + q * kCpThreads;
-        if (j < tn) skey[j + 1] = kr[q];
-      }
-      if (threadIdx.x == 0) skey[0] = prev;
+      for (int q = 0; q < kDdKeys; q++) keep[q] &= !hit[q];
     }
-    __syncthreads();
-    uint32_t bits = 0;
-    if (j0 < tn) {
-      uint32_t p = 0;
-      uint64_t g = f0;  // unstaged slice: this thread's position in FULL
-      if (staged && len) {
-        const uint64_t k0 = sel.expand(skey[j0 + 1]);
-        uint32_t lo = 0, hi = len;
-        while (lo < hi) {
-          const uint32_t mid = (lo + hi) >> 1;
-          if (stage[mid] < k0) lo = mid + 1;
-          else hi = mid;
-        }
-        p = lo;
-      }
+    if (sel.n_head) {
+      dd_lower_bounds(sel.head, sel.n_head, k, hit);
 #pragma unroll
-      for (int q = 0; q < kCpItems; q++) {
-        const uint32_t j = j0 + q;
-        if (j >= tn) break;
-        const K c = skey[j + 1];
-        bool keep = !(sel.dedup && (tile + j) > 0 && skey[j] == c);
-        if (keep && len) {
-          const uint64_t k = sel.expand(c);
-          if (staged) {
-            while (p < len && stage[p] < k) p++;
-            keep = !(p < len && stage[p] == k);
-          } else {
-            g = q == 0 ? lower_bound_u64(sel.full, f0, f1, k)
-                       : gallop_lower_bound_u64(sel.full, g, f1, k);
-            keep = !(g < f1 && sel.full[g] == k);
-          }
-        }
-        if (keep && h1 > h0) {
-          const uint64_t k = sel.expand(c);
-          const uint64_t g = lower_bound_u64(sel.head, h0, h1, k);
-          keep = !(g < h1 && sel.head[g] == k);
-        }
-        bits |= (keep ? 1u : 0u) << q;
-      }
+      for (int q = 0; q < kDdKeys; q++) keep[q] &= !hit[q];
     }
-    // lanes 4w..4w+3 hold the bytes of flag word w of this warp's 128 keys
-    uint32_t word = bits << (8 * (lane & 3));
-    word |= __shfl_down_sync(kAllLanes, word, 1);
-    word |= __shfl_down_sync(kAllLanes, word, 2);
-    if ((lane & 3) == 0 && j0 < tn) flags[(tile + j0) / 32] = word;
-    cnt += __popc(bits);
-    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kDdKeys; q++) {
+      const uint32_t m = __ballot_sync(kAllLanes, keep[q]);
+      if (lane == 0 && w0 + q * 32 < end) flags[(w0 + q * 32) / 32] = m;
+      cnt += __popc(m);
+    }
   }
   uint32_t tot;
-  block_excl_scan(cnt, sh, &tot);
+  block_excl_scan(lane == 0 ? cnt : 0u, sh, &tot);
   if (threadIdx.x == 0) blk_counts[blockIdx.x] = tot;
 }
 
@@ -407,19 +315,6 @@ __device__ __forceinline__ uint64_t dm_path(const DedupDiffSel<K>& sel, uint64_t
 
 // split[t] = a-keys among the first t*kCpTile merged elements; hpos[t] = the
 // HEAD position of a[split[t]] (n_head past the last key).
-// Device loop (d_n set): the merge path and the probe path are both in the
-// graph and each kernel runs only when the counts on the device select its
-// path (FULL at most kDmMaxFullRatio times the keys: merge path).
-constexpr uint64_t kDmMaxFullRatio = 16;
-enum DiffPath : int { kPathAny = 0, kPathMerge = 1, kPathProbe = 2 };
-
-template <typename K>
-__device__ __forceinline__ bool diff_path_runs(int path, const DedupDiffSel<K>& sel, uint64_t n) {
-  if (path == kPathAny) return true;
-  const bool merge = sel.n_full <= kDmMaxFullRatio * n;
-  return (path == kPathMerge) == merge;
-}
-
 template <typename K>
 __global__ void dm_split_kernel(DedupDiffSel<K> sel, uint64_t na, uint64_t tiles,
                                 uint64_t* __restrict__ split, uint64_t* __restrict__ hpos,
@@ -586,69 +481,48 @@ static __global__ void __launch_bounds__(kCpThreads) cp_count_kernel(const uint3
   if (threadIdx.x == 0) blk_counts[blockIdx.x] = tot;
 }
 
-// The merge-path pass streams all of FULL; past kDmMaxFullRatio the per-tile
-// probes of dd_flag_kernel read less.
-
 // compact() for DedupDiffSel with a FULL array: merge path when FULL is not
-// much larger than the keys, tiled shared-memory probes otherwise.
+// much larger than the keys, one search per key otherwise.
 template <typename K>
 void compact_diff(const Launch& L, DedupDiffSel<K> sel, uint64_t n, uint64_t* d_total, Scratch& s) {
   if (!sel.head || sel.n_head == 0) {
     sel.head = nullptr;
     sel.n_head = 0;
   }
-  if ((!sel.full || sel.n_full == 0) && !sel.head) {
-    compact(L, sel, n, d_total, s);
-    return;
-  }
   if (!sel.full) sel.n_full = 0;
-  if (n == 0) {
-    SRDL_CUDA(cudaMemsetAsync(d_total, 0, sizeof(uint64_t), L.stream));
+  if ((sel.n_full == 0 && !sel.head) || n == 0) {
+    compact(L, sel, n, d_total, s);
     return;
   }
   const uint64_t chunk = cp_chunk(n, L.num_sms);
   const int nb = cp_blocks(n, chunk);
-  const uint64_t tiles = (n + kCpTile - 1) / kCpTile;
   uint32_t* flags = s.take<uint32_t>(cp_words(n));
   uint32_t* counts = s.take<uint32_t>(nb);
-  if (sel.n_full <= kDmMaxFullRatio * n) {
+  if (sel.n_full && sel.n_full <= kDmMaxFullRatio * n) {
     const uint64_t mtiles = (n + sel.n_full + kCpTile - 1) / kCpTile;
     SRDL_REQUIRE(mtiles < (1ull << 31), kErrCapacity, "set difference: too many rows");
     uint64_t* split = s.take<uint64_t>(mtiles + 1);
     uint64_t* mhpos = sel.head ? s.take<uint64_t>(mtiles + 1) : nullptr;
     SRDL_CUDA(cudaMemsetAsync(flags, 0, cp_words(n) * 4, L.stream));
-    dm_split_kernel<K><<<(unsigned)((mtiles + 1 + 255) / 256), 256, 0, L.stream>>>(sel, n, mtiles,
-                                                                                  split, mhpos, nullptr,
-                                                                                  kPathAny);
+    dm_split_kernel<K><<<(unsigned)((mtiles + 1 + 255) / 256), 256, 0, L.stream>>>(sel, n, mtiles, split, mhpos,
+                                                                                  nullptr, kPathAny);
     const unsigned mgrid = (unsigned)std::min<uint64_t>(mtiles, (uint64_t)L.num_sms * 4);
-    dm_mark_kernel<K><<<mgrid, kCpThreads, 0, L.stream>>>(sel, n, mtiles, split, mhpos, flags, nullptr,
-                                                          kPathAny);
+    dm_mark_kernel<K><<<mgrid, kCpThreads, 0, L.stream>>>(sel, n, mtiles, split, mhpos, flags, nullptr, kPathAny);
     cp_count_kernel<K><<<nb, kCpThreads, 0, L.stream>>>(flags, n, chunk, counts, sel, nullptr, kPathAny);
-    cp_write_kernel<DedupDiffSel<K>><<<nb, kCpThreads, 0, L.stream>>>(sel, n, chunk, flags, counts,
-                                                                       d_total, nullptr);
-    SRDL_CUDA(cudaGetLastError());
-    count_launches(4);
-    return;
+    count_launches(3);
+  } else {
+    dd_probe_kernel<K><<<nb, kCpThreads, 0, L.stream>>>(sel, n, chunk, flags, counts, nullptr, kPathAny);
+    count_launches(1);
   }
-  uint64_t* fpos = s.take<uint64_t>(tiles + 1);
-  uint64_t* hpos = sel.head ? s.take<uint64_t>(tiles + 1) : nullptr;
-  prefer_shared(dd_flag_kernel<K>);
-  const uint64_t bthreads = (tiles + 1) * 32;
-  dd_bounds_kernel<K><<<(unsigned)((bthreads + 255) / 256), 256, 0, L.stream>>>(sel, n, tiles, fpos,
-                                                                                hpos, nullptr, kPathAny);
-  dd_flag_kernel<K><<<nb, kCpThreads, 0, L.stream>>>(sel, n, chunk, fpos, hpos, flags, counts,
-                                                     nullptr, kPathAny);
-  cp_write_kernel<DedupDiffSel<K>><<<nb, kCpThreads, 0, L.stream>>>(sel, n, chunk, flags, counts,
-                                                                     d_total, nullptr);
+  cp_write_kernel<DedupDiffSel<K>><<<nb, kCpThreads, 0, L.stream>>>(sel, n, chunk, flags, counts, d_total, nullptr);
   SRDL_CUDA(cudaGetLastError());
-  count_launches(3);
+  count_launches(1);
 }
 
 // compact_diff with the key count on the device (device loop): `cap` keys
 // of room, *d_n of them present, FULL's count at sel.d_n_full (n_full its
-// capacity).  Both the merge path and the per-tile probe path are launched;
-// each kernel runs only when the counts on the device select its path (the
-// host's rule: merge while FULL is at most kDmMaxFullRatio times the keys),
+// capacity).  Both the merge path and the probe path are launched; each kernel
+// runs only when the counts on the device select its path (the host's rule),
 // so no host decision depends on the counts.  Grids are sized for the
 // capacities and each block derives its share of the true counts.
 inline size_t diff_dev_extra_bytes(uint64_t cap, uint64_t full_cap) {
@@ -669,32 +543,23 @@ void compact_diff_dev(const Launch& L, DedupDiffSel<K> sel, uint64_t cap, const 
   }
   const uint64_t chunk = cp_chunk(cap, L.num_sms);
   const int nb = cp_blocks(cap, chunk);
-  const uint64_t tiles = (cap + kCpTile - 1) / kCpTile;
   const uint64_t mtiles = (cap + sel.n_full + kCpTile - 1) / kCpTile;
   uint32_t* flags = s.take<uint32_t>(cp_words(cap));
   uint32_t* counts = s.take<uint32_t>(nb);
-  uint64_t* fpos = s.take<uint64_t>(tiles + 1);
   uint64_t* split = s.take<uint64_t>(mtiles + 1);
-  prefer_shared(dd_flag_kernel<K>);
   // merge path: the mark pass ORs its bits into zeroed flag words
   SRDL_CUDA(cudaMemsetAsync(flags, 0, cp_words(cap) * 4, L.stream));
-  dm_split_kernel<K><<<(unsigned)((mtiles + 1 + 255) / 256), 256, 0, L.stream>>>(sel, cap, mtiles, split,
-                                                                                nullptr, d_n, kPathMerge);
+  dm_split_kernel<K><<<(unsigned)((mtiles + 1 + 255) / 256), 256, 0, L.stream>>>(sel, cap, mtiles, split, nullptr,
+                                                                                d_n, kPathMerge);
   const unsigned mgrid = (unsigned)std::min<uint64_t>(mtiles, (uint64_t)L.num_sms * 4);
-  dm_mark_kernel<K><<<mgrid, kCpThreads, 0, L.stream>>>(sel, cap, mtiles, split, nullptr, flags, d_n,
-                                                        kPathMerge);
+  dm_mark_kernel<K><<<mgrid, kCpThreads, 0, L.stream>>>(sel, cap, mtiles, split, nullptr, flags, d_n, kPathMerge);
   cp_count_kernel<K><<<nb, kCpThreads, 0, L.stream>>>(flags, cap, 0, counts, sel, d_n, kPathMerge);
-  // probe path (a capped grid of warps walks the tile boundaries)
-  const uint64_t bthreads = (tiles + 1) * 32;
-  const uint64_t bblocks = std::min<uint64_t>((bthreads + 255) / 256, (uint64_t)L.num_sms * 8);
-  dd_bounds_kernel<K><<<(unsigned)bblocks, 256, 0, L.stream>>>(sel, cap, tiles, fpos, nullptr, d_n,
-                                                              kPathProbe);
-  dd_flag_kernel<K><<<nb, kCpThreads, 0, L.stream>>>(sel, cap, 0, fpos, nullptr, flags, counts, d_n,
-                                                     kPathProbe);
+  // probe path
+  dd_probe_kernel<K><<<nb, kCpThreads, 0, L.stream>>>(sel, cap, 0, flags, counts, d_n, kPathProbe);
   // either way: the ordered write of the kept keys
   cp_write_kernel<DedupDiffSel<K>><<<nb, kCpThreads, 0, L.stream>>>(sel, cap, 0, flags, counts, d_total, d_n);
   SRDL_CUDA(cudaGetLastError());
-  count_launches(6);
+  count_launches(5);
 }
 
 // Distinct first-column values of a sorted key array.

@@ -371,7 +371,6 @@ static void warm_sort_kernels() {
   prefer_shared(rs_scatter<K, 6>);
   prefer_shared(rs_scatter<K, 7>);
   prefer_shared(rs_scatter<K, 8>);
-  prefer_shared(dd_flag_kernel<K>);
 }
 
 void warm_device_loop_kernels(int bits) {

@@ -8,10 +8,24 @@ import pytest
 from conftest import load_plan
 from srdatalog_b200 import native
 from srdatalog_b200 import workloads as W
-from test_gpu_primitives import gpu_merge, keys_with_bits
+from test_gpu_primitives import gpu_diff, gpu_merge, keys_with_bits
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip('torch')
+
+TOP = np.uint64(0xFFFFFFFFFFFFFFFF)
+
+
+@pytest.mark.parametrize('na,nb', [(1, 4), (2047, 2049), (2048, 2048), (31, 6000), (4096, 4096 * 16),
+                                   (4096, 4096 * 16 + 1), (20_481, 700_000), (1_300_000, 2)])
+def test_set_difference_tile_edges(na, nb):
+  rng = np.random.default_rng(na + nb)
+  u = np.unique(np.concatenate([keys_with_bits(rng, na + nb, 32), np.array([0, TOP], np.uint64)]))
+  a = np.sort(rng.choice(u, min(na, len(u)), replace=False))
+  b = np.sort(rng.choice(u, min(nb, len(u)), replace=False))
+  a[0], a[-1] = u[0], u[-1]   # the smallest and the largest key there is
+  for bb in (b, np.unique(np.append(b, u[0])), np.unique(np.append(b, u[-1])), b[b > a[len(a) // 2]]):
+    assert np.array_equal(gpu_diff(a, bb), oracle.set_difference(a, bb))
 
 
 @pytest.mark.parametrize('na,nb', [(1, 2047), (2048, 0), (2048, 2048), (2049, 4095), (1, 2_000_000),
