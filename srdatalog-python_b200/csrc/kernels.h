@@ -15,7 +15,7 @@ struct Launch {
   cudaStream_t stream = 0;
   int num_sms = 148;
   uint32_t* d_err = nullptr;  // device error word (bounded-wait failures etc.)
-  int radix_bits = 8;         // widest radix-sort digit (1..8): passes = ceil(key bits / this)
+  int radix_bits = 8;         // widest radix-sort digit (1..7; 8: the sort's own choice)
   int join_bpsm = 16;         // join launches: at most this many blocks per SM (work per warp)
   int join_chunk = 4096;      // two-source column join: largest chunk of candidates a warp takes
 };
@@ -59,6 +59,9 @@ void max_u32(const Launch& L, const uint32_t* d, uint64_t n, uint32_t* d_max);
 // ---------------------------------------------------------------- sort
 // Bits needed to hold every value of the active domain (max value < 2^bits).
 int value_bits(uint32_t max_value);
+
+// Counting passes the sort makes over keys of two dom_bits halves.
+int radix_passes(const Launch& L, int dom_bits);
 
 // Scratch needed by sort_dedup for n input keys.
 size_t sort_scratch_bytes(uint64_t n, int dom_bits);

@@ -464,8 +464,7 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
                       &X.ctl_d()->bodies, loop_marks_);
     }
     const int ks = 2 * bits_ <= 32 ? 4 : 8;
-    const int maxw = L_.radix_bits >= 1 && L_.radix_bits <= 8 ? L_.radix_bits : 8;
-    const int passes = (2 * bits_ + maxw - 1) / maxw;
+    const int passes = radix_passes(L_, bits_);
     loop_ctrl_kernel<<<1, 32, 0, L_.stream>>>(X.ctl_d(), cnt, (int)X.rels.size(), p, ks, passes, hw, hi,
                                               set_if);
     SRDL_CUDA(cudaGetLastError());

@@ -728,7 +728,7 @@ void Database::sort_into(Index& out, const uint64_t* in, uint64_t n, bool swap, 
     // keys and writes the distinct ones (plus one probe word per key into
     // FULL when the delta is fused).
     const double ks = 2 * kb <= 32 ? 4 : 8;
-    const double passes = (2 * kb + L_.radix_bits - 1) / L_.radix_bits;
+    const double passes = radix_passes(L_, kb);
     kev_[pid].bytes = passes * 2 * ks * n + 8.0 * n + ks * n + ks * n + 8.0 * out.n +
                       (diff ? 8.0 * n : 0);
   }

@@ -9,26 +9,35 @@
 // Design.  Datalog creates no values: every value of every relation comes
 // from the loaded inputs (and rule constants), so the runtime knows a bound
 // 2^bits on all values.  A two-column key (hi, lo) is compressed to
-// (hi << bits) | lo -- 32 bits when 2*bits <= 32 -- and sorted with
-// ceil(2*bits / 8) stable counting passes (digits of at most Launch::radix_bits).  Each pass is a histogram launch
-// (shared-memory counters per block), a per-digit scan over the blocks, and a
-// scatter launch in which every warp ranks its keys with one ballot per digit
-// bit, the tile is staged in shared memory in digit order and written out
-// coalesced.  No
-// block ever waits on another.  The dedup (and optional "not in FULL" test)
-// runs as one order-preserving compaction over the sorted keys that also
-// expands them back to (hi << 32) | lo.
+// (hi << bits) | lo -- 32 bits when 2*bits <= 32 -- and sorted with stable
+// counting passes over digits of at most kRsAutoBits bits (or the caller's
+// Launch::radix_bits).  Each pass is a histogram launch (shared-memory counters
+// per block), a per-digit scan over the blocks, and a scatter launch in which
+// every warp ranks its keys with one ballot per digit bit, the tile is staged
+// in shared memory in digit order and written out coalesced; the first pass
+// reads the caller's keys and packs them on the way.  No block ever waits on
+// another.  The dedup (and optional "not in FULL" test) runs as one
+// order-preserving compaction over the sorted keys that also expands them back
+// to (hi << 32) | lo.  Up to kRsSmall keys take one launch of one block.
+#include <atomic>
+#include <type_traits>
+
 #include "compact.cuh"
 #include "kernels.h"
 
 namespace srdl {
 
-constexpr int kRsThreads = 256;
+constexpr int kRsThreads = 512;
 constexpr int kRsWarps = kRsThreads / 32;
-constexpr int kRsPerWarp = 256;                  // keys per warp per tile
-constexpr int kRsTile = kRsWarps * kRsPerWarp;   // 2048 keys per tile
-constexpr int kRsBins = 256;
-static_assert(kRsThreads == kRsBins, "one thread per digit in the per-tile digit loops");
+constexpr int kRsItems = 16;                     // keys per thread and tile, at most
+constexpr int kRsTile = kRsThreads * kRsItems;   // 8192 keys per tile, at most
+constexpr int kRsMinChunk = 2048;                // keys a block takes, at least
+constexpr int kRsMaxBits = 9;                    // widest digit there is a kernel for
+constexpr int kRsBlocksPerSm = 2;                // resident blocks
+// Widest digit when the caller names none: 100M keys of 42 bits take 3.99 ms in
+// five passes of at most 9 bits; with digits of 8 bits the sixth pass made them
+// 8% slower, and a 10-bit digit's counters leave one block per SM.
+constexpr int kRsAutoBits = 9;
 
 int value_bits(uint32_t max_value) {
   int b = 0;
@@ -36,56 +45,83 @@ int value_bits(uint32_t max_value) {
   return b ? b : 1;
 }
 
+// A key of the caller's array, (hi << 32) | lo, in packed form.
 template <typename K>
-__global__ void rs_pack(const uint64_t* __restrict__ in, uint64_t n, int bits, bool swap,
-                        K* __restrict__ out, const uint64_t* d_n) {
-  n = dev_size(n, d_n);
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    uint64_t k = in[i];
-    uint64_t hi = k >> 32, lo = k & 0xffffffffull;
-    if (swap) {
-      uint64_t t = hi;
-      hi = lo;
-      lo = t;
-    }
-    out[i] = (K)((hi << bits) | lo);
+__device__ __forceinline__ K rs_packed(uint64_t k, int bits, bool swap) {
+  uint64_t hi = k >> 32, lo = k & 0xffffffffull;
+  if (swap) {
+    const uint64_t t = hi;
+    hi = lo;
+    lo = t;
   }
+  return (K)((hi << bits) | lo);
 }
 
-template <typename K>
-__global__ void __launch_bounds__(kRsThreads) rs_hist(const K* __restrict__ keys, uint64_t n,
-                                                      uint64_t chunk, int shift, int nbins,
-                                                      uint32_t* __restrict__ counts,
-                                                      const uint64_t* d_n) {
-  __shared__ uint32_t h[kRsBins];
+// Keys per block when nb blocks share n: an even split in multiples of 512 (the
+// histogram's 16-byte loads start there), kRsMinChunk at least.
+__host__ __device__ __forceinline__ uint64_t rs_chunk(uint64_t n, uint64_t nb) {
+  const uint64_t c = ((n + nb - 1) / nb + 511) & ~uint64_t(511);
+  return c < (uint64_t)kRsMinChunk ? (uint64_t)kRsMinChunk : c;
+}
+
+// Digit counts of every block's chunk, digit-major.  The first pass (FIRST)
+// reads the caller's keys and packs them on the way.
+template <typename K, bool FIRST>
+__global__ void __launch_bounds__(kRsThreads) rs_hist(const void* __restrict__ in, uint64_t n, uint64_t chunk,
+                                                      int shift, int nbins, uint32_t* __restrict__ counts,
+                                                      const uint64_t* d_n, int bits, bool swap) {
+  __shared__ uint32_t h[1 << kRsMaxBits];
   n = dev_size(n, d_n);
-  chunk = dev_chunk(chunk, n, kRsTile);
+  if (d_n) chunk = rs_chunk(n, gridDim.x);
   for (int d = threadIdx.x; d < nbins; d += kRsThreads) h[d] = 0;
   __syncthreads();
   const uint64_t begin = (uint64_t)blockIdx.x * chunk;
   const uint64_t end = begin + chunk < n ? begin + chunk : n;
   const uint32_t mask = nbins - 1;
-  // 16-byte loads: the chunk starts a multiple of kRsTile keys into a
-  // 256-byte aligned array; a ragged tail is read key by key.
-  constexpr uint64_t kPer = 16 / sizeof(K);
-  const uint64_t vend = begin < end ? begin + (end - begin) / kPer * kPer : begin;
-  const uint4* vec = reinterpret_cast<const uint4*>(keys + begin);
-  for (uint64_t q = threadIdx.x; begin + q * kPer < vend; q += kRsThreads) {
-    const uint4 v = __ldg(vec + q);
-    if constexpr (sizeof(K) == 8) {
-      const uint64_t k0 = ((uint64_t)v.y << 32) | v.x, k1 = ((uint64_t)v.w << 32) | v.z;
-      atomicAdd(&h[(uint32_t)(k0 >> shift) & mask], 1u);
-      atomicAdd(&h[(uint32_t)(k1 >> shift) & mask], 1u);
-    } else {
-      atomicAdd(&h[(v.x >> shift) & mask], 1u);
-      atomicAdd(&h[(v.y >> shift) & mask], 1u);
-      atomicAdd(&h[(v.z >> shift) & mask], 1u);
-      atomicAdd(&h[(v.w >> shift) & mask], 1u);
+  if constexpr (FIRST) {
+    // 8-byte loads: the caller's array is only that aligned
+    const uint64_t* raw = static_cast<const uint64_t*>(in);
+    uint64_t i = begin + threadIdx.x;
+    for (; i + 3 * kRsThreads < end; i += 4 * kRsThreads) {
+      uint64_t k[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) k[q] = __ldg(raw + i + q * kRsThreads);
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        atomicAdd(&h[(uint32_t)(rs_packed<K>(k[q], bits, swap) >> shift) & mask], 1u);
     }
+    for (; i < end; i += kRsThreads)
+      atomicAdd(&h[(uint32_t)(rs_packed<K>(__ldg(raw + i), bits, swap) >> shift) & mask], 1u);
+  } else {
+    // 16-byte loads: the chunk starts a multiple of 512 keys into a 256-byte
+    // aligned array; a ragged tail is read key by key.
+    const K* keys = static_cast<const K*>(in);
+    constexpr uint64_t kPer = 16 / sizeof(K);
+    const uint64_t vend = begin < end ? begin + (end - begin) / kPer * kPer : begin;
+    const uint4* vec = reinterpret_cast<const uint4*>(keys + begin);
+    auto add = [&](const uint4& v) {
+      if constexpr (sizeof(K) == 8) {
+        const uint64_t k0 = ((uint64_t)v.y << 32) | v.x, k1 = ((uint64_t)v.w << 32) | v.z;
+        atomicAdd(&h[(uint32_t)(k0 >> shift) & mask], 1u);
+        atomicAdd(&h[(uint32_t)(k1 >> shift) & mask], 1u);
+      } else {
+        atomicAdd(&h[(v.x >> shift) & mask], 1u);
+        atomicAdd(&h[(v.y >> shift) & mask], 1u);
+        atomicAdd(&h[(v.z >> shift) & mask], 1u);
+        atomicAdd(&h[(v.w >> shift) & mask], 1u);
+      }
+    };
+    const uint64_t nv = begin < end ? (vend - begin) / kPer : 0;
+    uint64_t q = threadIdx.x;
+    for (; q + kRsThreads < nv; q += 2 * kRsThreads) {
+      const uint4 v0 = __ldg(vec + q), v1 = __ldg(vec + q + kRsThreads);
+      add(v0);
+      add(v1);
+    }
+    if (q < nv) add(__ldg(vec + q));
+    for (uint64_t i = vend + threadIdx.x; i < end; i += kRsThreads)
+      atomicAdd(&h[(uint32_t)(keys[i] >> shift) & mask], 1u);
   }
-  for (uint64_t i = vend + threadIdx.x; i < end; i += kRsThreads)
-    atomicAdd(&h[(uint32_t)(keys[i] >> shift) & mask], 1u);
   __syncthreads();
   for (int d = threadIdx.x; d < nbins; d += kRsThreads) counts[(uint64_t)d * gridDim.x + blockIdx.x] = h[d];
 }
@@ -93,11 +129,13 @@ __global__ void __launch_bounds__(kRsThreads) rs_hist(const K* __restrict__ keys
 // Block d turns row d of the digit-major counters (one counter per
 // histogram block) into exclusive offsets within the digit, in place, and
 // writes the digit's total to digit_tot[d].
-__global__ void __launch_bounds__(kRsThreads) rs_rowscan(uint32_t* c, int nb,
-                                                         uint32_t* __restrict__ digit_tot) {
-  __shared__ uint32_t sh[kRsThreads / 32 + 1];
+constexpr int kRsScanThreads = 256;
+
+__global__ void __launch_bounds__(kRsScanThreads) rs_rowscan(uint32_t* c, int nb,
+                                                             uint32_t* __restrict__ digit_tot) {
+  __shared__ uint32_t sh[kRsScanThreads / 32 + 1];
   uint32_t* row = c + (uint64_t)blockIdx.x * nb;
-  const int per = (nb + kRsThreads - 1) / kRsThreads;
+  const int per = (nb + kRsScanThreads - 1) / kRsScanThreads;
   const int s = threadIdx.x * per, e = min(nb, s + per);
   uint32_t sum = 0;
   for (int i = s; i < e; i++) sum += row[i];
@@ -111,180 +149,258 @@ __global__ void __launch_bounds__(kRsThreads) rs_rowscan(uint32_t* c, int nb,
   if (threadIdx.x == 0) digit_tot[blockIdx.x] = tot;
 }
 
-// Asynchronous 16-byte global -> shared copy (cp.async, no registers held);
-// bytes past `src_bytes` (< 16 on a ragged tail) are zero-filled.
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, uint32_t src_bytes) {
-  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem),
-               "r"(src_bytes)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() {
-  asm volatile("cp.async.commit_group;\n" ::: "memory");
-}
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-
-// Issue the copy of keys [tile, min(tile + kRsTile, end)) into `buf`.  Tile
-// starts are multiples of kRsTile keys from a 256-byte aligned buffer, so
-// every 16-byte piece is aligned; a piece that straddles `end` copies only
-// the valid bytes, and pieces past it copy nothing.
-template <typename K>
-__device__ __forceinline__ void rs_prefetch(K* buf, const K* in, uint64_t tile, uint64_t end) {
-  constexpr int kPieces = kRsTile * (int)sizeof(K) / 16;
-  const uint64_t valid_bytes = (end > tile ? end - tile : 0) * sizeof(K);
-  const char* src = reinterpret_cast<const char*>(in + tile);
-  char* dst = reinterpret_cast<char*>(buf);
-  for (int p = threadIdx.x; p < kPieces; p += kRsThreads) {
-    const uint64_t off = (uint64_t)p * 16;
-    const uint64_t left = off >= valid_bytes ? 0 : valid_bytes - off;
-    const uint32_t nb = left < 16 ? (uint32_t)left : 16u;
-    cp_async16(dst + off, nb ? src + off : src, nb);
-  }
-  cp_async_commit();
-}
-
-// One counting pass over this block's chunk, a tile of kRsTile keys at a
-// time, for digits of DB bits.  The next tile is copied into the other shared
-// buffer while the current one is ranked and written, so every block keeps a
-// tile of loads in flight.  Within a warp, the lanes holding the same digit
-// are found with DB ballots (one per digit bit), which is cheaper than a
-// match instruction; the lowest such lane adds the group's size to the warp's
-// counter for the digit and passes the old value on.  The staged
-// (digit-ordered) tile reuses the buffer the current keys were read from.
-// Five resident blocks per SM (their shared memory fits; the register cap
-// that needs costs no spills).
+// Shared memory of a scatter block: the staged tile, a 16-bit counter per
+// warp and digit, and per digit the next output position and its offset from
+// the staged position.
 template <typename K, int DB>
-__global__ void __launch_bounds__(kRsThreads, 5) rs_scatter(const K* __restrict__ in,
-                                                         K* __restrict__ out, uint64_t n,
-                                                         uint64_t chunk, int shift,
-                                                         const uint32_t* __restrict__ offs,
-                                                         const uint32_t* __restrict__ digit_tot,
-                                                         const uint64_t* d_n) {
+constexpr size_t rs_smem_bytes() {
+  constexpr size_t bins = 1 << DB;
+  return kRsTile * sizeof(K) + kRsWarps * (bins < 8 ? 16 : bins * 2) + 2 * (bins < 4 ? 16 : bins * 4);
+}
+
+// Lanes of the warp whose digit equals this lane's: one ballot per digit bit.
+// Written in PTX because the same loop in C++ compiled to eight instructions
+// per bit instead of four, and the integer pipe they use bounds the pass.
+template <int DB>
+__device__ __forceinline__ unsigned rs_peers(uint32_t d) {
+  unsigned peers = kAllLanes;
+#pragma unroll
+  for (int b = 0; b < DB; b++)
+    asm volatile(
+        "{\n"
+        "  .reg .pred p;\n"
+        "  .reg .b32 t;\n"
+        "  setp.ne.u32 p, %1, 0;\n"
+        "  vote.sync.ballot.b32 t, p, 0xffffffff;\n"
+        "  @!p not.b32 t, t;\n"
+        "  and.b32 %0, %0, t;\n"
+        "}\n"
+        : "+r"(peers)
+        : "r"(d & (1u << b)));
+  return peers;
+}
+
+// Stable rank of each lane's digit among the earlier keys of its warp with the
+// same digit; counter[d] holds the warp's keys of digit d so far.  The highest
+// lane of a digit stores the new count, which it knows from its own rank.
+// (Setting lane bits in a shared match mask instead of the ballots takes fewer
+// instructions but 40 instead of 27 shared-memory wavefronts per 32 keys.)
+template <int DB>
+__device__ __forceinline__ uint32_t rs_rank(uint16_t* counter, uint32_t d, unsigned lt, unsigned gt) {
+  const unsigned peers = rs_peers<DB>(d);
+  const uint32_t rank = counter[d] + __popc(peers & lt);
+  __syncwarp();
+  if (!(peers & gt)) counter[d] = (uint16_t)(rank + 1);
+  __syncwarp();
+  return rank;
+}
+
+// One counting pass over this block's chunk, a tile of at most kRsTile keys at
+// a time, for digits of DB bits.
+//
+// A warp owns 32 * rounds consecutive keys of the tile, 32 per round, held in
+// registers, and ranks them with rs_rank.  Two digits' counters share a word:
+// one thread per word turns the warps' counts into staged positions, one block
+// scan orders the digits.  The keys are then staged in digit order and, while
+// the next tile's keys are being loaded into the registers they left, written
+// out in runs.  Full tiles of 16 keys per thread take a path without bounds
+// checks.
+//
+// Bound: integer operations, which issue every other cycle, and shared-memory
+// wavefronts (each about half used: two blocks of 16 warps share an SM);
+// 16 keys per thread spread the per-digit work over 8192 keys and keep a tile's
+// runs at 128 bytes for 9-bit digits.  100M keys of 42 bits: 0.58 ms per 9-bit
+// pass, against 0.60 ms per 7-bit pass with 2048-key tiles and the ballots
+// compiled from C++.  Tiles of 6144 keys with three blocks per SM, tiles of 4096
+// with four, and rounds ranked four at a time were 7%, 8% and 3% slower.  Keys
+// past the end are all ones: they rank behind every real key and are not
+// written.
+template <typename K, int DB, bool FIRST>
+__global__ void __launch_bounds__(kRsThreads, 2) rs_scatter(const void* __restrict__ in, K* __restrict__ out,
+                                                            uint64_t n, uint64_t chunk, int shift,
+                                                            const uint32_t* __restrict__ offs,
+                                                            const uint32_t* __restrict__ digit_tot,
+                                                            const uint64_t* d_n, int bits, bool swap) {
   constexpr int nbins = 1 << DB;
   constexpr uint32_t mask = nbins - 1;
-  __shared__ uint32_t base[kRsBins];             // next global output position per digit
-  __shared__ uint32_t gofs[kRsBins];             // base[d] minus the digit's start in the staged tile
-  __shared__ uint32_t wofs[kRsWarps][kRsBins];   // per-warp digit counts -> staged positions
-  __shared__ uint32_t scan_sh[kRsThreads / 32 + 1];
-  __shared__ __align__(16) K buf[2][kRsTile];
+  constexpr int pairs = nbins / 2;                 // words holding two counters
+  constexpr int stride = pairs < 4 ? 4 : pairs;    // words per warp
+  extern __shared__ __align__(16) unsigned char rs_sm[];
+  K* buf = reinterpret_cast<K*>(rs_sm);
+  uint32_t* cnt = reinterpret_cast<uint32_t*>(rs_sm + kRsTile * sizeof(K));
+  uint32_t* base = cnt + kRsWarps * stride;        // next global output position per digit
+  uint32_t* gofs = base + (nbins < 4 ? 4 : nbins); // base minus the digit's start in the staged tile
+  __shared__ uint32_t scan_sh[kRsWarps + 1];
+  static_assert(pairs <= kRsThreads, "one thread per counter word");
 
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   n = dev_size(n, d_n);
-  chunk = dev_chunk(chunk, n, kRsTile);
+  if (d_n) chunk = rs_chunk(n, gridDim.x);
   const uint64_t begin = (uint64_t)blockIdx.x * chunk;
   const uint64_t end = begin + chunk < n ? begin + chunk : n;
-  if (begin < end) rs_prefetch(buf[0], in, begin, end);
+  if (begin >= end) return;
+  const uint32_t len = (uint32_t)(end - begin);
+  const uint32_t ntiles = (len + kRsTile - 1) / kRsTile;
+  // equal tiles: rounds <= kRsItems
+  const int rounds = (int)((len + ntiles * kRsThreads - 1) / (ntiles * kRsThreads));
+  const uint32_t tile_keys = (uint32_t)rounds * kRsThreads;
+
+  K key[kRsItems];
+  auto fetch = [&](uint64_t i) -> K {
+    if constexpr (FIRST) return rs_packed<K>(__ldg(static_cast<const uint64_t*>(in) + i), bits, swap);
+    else return __ldg(static_cast<const K*>(in) + i);
+  };
+  auto load = [&](uint64_t tile) {
+    const uint64_t i0 = tile + (uint32_t)(wid * rounds * 32 + lane);
+    if (rounds == kRsItems && tile + kRsTile <= end) {
+#pragma unroll
+      for (int r = 0; r < kRsItems; r++) key[r] = fetch(i0 + r * 32);
+      return;
+    }
+#pragma unroll
+    for (int r = 0; r < kRsItems; r++) {
+      key[r] = ~K(0);
+      if (r < rounds && i0 + r * 32 < end) key[r] = fetch(i0 + r * 32);
+    }
+  };
+  load(begin);
   {
     // digit base = keys with a smaller digit; plus this block's offset in the digit
-    const int d = threadIdx.x;  // kRsThreads == kRsBins
-    const uint32_t t = d < nbins ? digit_tot[d] : 0;
+    const int t = threadIdx.x;
+    const uint32_t t0 = t < pairs ? digit_tot[2 * t] : 0, t1 = t < pairs ? digit_tot[2 * t + 1] : 0;
     uint32_t all;
-    const uint32_t dbase = block_excl_scan(t, scan_sh, &all);
-    base[d] = d < nbins ? dbase + offs[(uint64_t)d * gridDim.x + blockIdx.x] : 0;
-  }
-
-  const unsigned lt = lanemask_lt();
-  int cur = 0;
-  for (uint64_t tile = begin; tile < end; tile += kRsTile, cur ^= 1) {
-#pragma unroll
-    for (int w = 0; w < kRsWarps; w++) wofs[w][threadIdx.x] = 0;
-    const uint64_t next = tile + kRsTile;
-    if (next < end) {
-      rs_prefetch(buf[cur ^ 1], in, next, end);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
+    const uint32_t db = block_excl_scan(t0 + t1, scan_sh, &all);
+    if (t < pairs) {
+      base[2 * t] = db + offs[(uint64_t)(2 * t) * gridDim.x + blockIdx.x];
+      base[2 * t + 1] = db + t0 + offs[(uint64_t)(2 * t + 1) * gridDim.x + blockIdx.x];
     }
-    __syncthreads();
-    const uint32_t cnt = (uint32_t)((end - tile) < kRsTile ? (end - tile) : kRsTile);
-    K key[kRsPerWarp / 32];
-    uint32_t rank[kRsPerWarp / 32];  // rank in the warp's digit run | digit << 16
-    // Warp `wid` owns keys [wid*256, +256) of the tile in rounds of 32, so the
-    // (round, lane) order is the input order.  Each round's counter update
-    // precedes the next round's (__syncwarp orders them): ranks are stable.
+  }
+  const unsigned lt = lanemask_lt(), gt = ~(lt | (1u << lane));
+  uint32_t* my = cnt + wid * stride;
+  uint16_t* my16 = reinterpret_cast<uint16_t*>(my);
+  for (uint64_t tile = begin; tile < end; tile += tile_keys) {
+    const uint32_t count = (uint32_t)(end - tile < tile_keys ? end - tile : tile_keys);
+    for (int i = lane; i < stride; i += 32) my[i] = 0;
+    __syncwarp();
+    uint32_t rank[kRsItems / 2];  // two 16-bit ranks within the warp's digit run per word
 #pragma unroll
-    for (int r = 0; r < kRsPerWarp / 32; r++) {
-      const uint32_t j = (uint32_t)wid * kRsPerWarp + r * 32 + lane;
-      const bool valid = j < cnt;
-      key[r] = buf[cur][j];
-      const uint32_t d = (uint32_t)(key[r] >> shift) & mask;
-      unsigned peers = __ballot_sync(kAllLanes, valid);
-#pragma unroll
-      for (int b = 0; b < DB; b++) {
-        const bool bit = (d >> b) & 1u;
-        const unsigned m = __ballot_sync(kAllLanes, bit);
-        peers &= bit ? m : ~m;
+    for (int r = 0; r < kRsItems; r++) {
+      if (r < rounds) {
+        const uint32_t rk = rs_rank<DB>(my16, (uint32_t)(key[r] >> shift) & mask, lt, gt);
+        rank[r / 2] = r & 1 ? rank[r / 2] | (rk << 16) : rk;
       }
-      // invalid lanes (a ragged last tile) get an empty group and lane 0 as leader
-      peers = valid ? peers : 0u;
-      const int leader = valid ? __ffs(peers) - 1 : 0;
-      uint32_t old = 0;
-      if (valid && lane == leader) old = atomicAdd(&wofs[wid][d], (uint32_t)__popc(peers));
-      old = __shfl_sync(kAllLanes, old, leader);
-      rank[r] = valid ? (old + __popc(peers & lt)) | (d << 16) : 0xffffffffu;
-      __syncwarp();
     }
     __syncthreads();
     // Per digit: staged start of each warp's run (tile start of the digit plus
     // the earlier warps' counts), and the global offset of the digit's run.
     {
-      const int d = threadIdx.x;  // kRsThreads == kRsBins
-      uint32_t c[kRsWarps], run = 0;
+      const int t = threadIdx.x;
+      uint32_t run = 0;
+      if (t < pairs) {
 #pragma unroll
-      for (int w = 0; w < kRsWarps; w++) {
-        c[w] = wofs[w][d];
-        run += c[w];
+        for (int w = 0; w < kRsWarps; w++) {
+          const uint32_t v = cnt[w * stride + t];
+          cnt[w * stride + t] = run;
+          run += v;  // (both halves stay below 2^16: a tile has 8192 keys)
+        }
       }
+      const uint32_t c0 = run & 0xffffu, c1 = run >> 16;
       uint32_t all;
-      uint32_t start = block_excl_scan(run, scan_sh, &all);
-      gofs[d] = base[d] - start;
-      base[d] += run;
+      const uint32_t start = block_excl_scan(c0 + c1, scan_sh, &all);
+      if (t < pairs) {
+        const uint32_t b0 = base[2 * t], b1 = base[2 * t + 1];
+        gofs[2 * t] = b0 - start;
+        gofs[2 * t + 1] = b1 - (start + c0);
+        base[2 * t] = b0 + c0;
+        base[2 * t + 1] = b1 + c1;
+        const uint32_t add = start | ((start + c0) << 16);
 #pragma unroll
-      for (int w = 0; w < kRsWarps; w++) {
-        wofs[w][d] = start;
-        start += c[w];
+        for (int w = 0; w < kRsWarps; w++) cnt[w * stride + t] += add;
       }
     }
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < kRsPerWarp / 32; r++) {
-      if (rank[r] != 0xffffffffu) buf[cur][wofs[wid][rank[r] >> 16] + (rank[r] & 0xffffu)] = key[r];
+    for (int r = 0; r < kRsItems; r++) {
+      if (r < rounds) {
+        const uint32_t rk = r & 1 ? rank[r / 2] >> 16 : rank[r / 2] & 0xffffu;
+        buf[my16[(uint32_t)(key[r] >> shift) & mask] + rk] = key[r];
+      }
     }
     __syncthreads();
-    for (uint32_t j = threadIdx.x; j < cnt; j += kRsThreads) {
-      const K k = buf[cur][j];
-      out[gofs[(uint32_t)(k >> shift) & mask] + j] = k;
+    if (tile + tile_keys < end) load(tile + tile_keys);
+    // (the next tile's stores into buf and gofs come after its first barrier)
+    if (count == kRsTile) {
+#pragma unroll
+      for (int q = 0; q < kRsItems; q++) {
+        const K k = buf[threadIdx.x + q * kRsThreads];
+        out[gofs[(uint32_t)(k >> shift) & mask] + (threadIdx.x + q * kRsThreads)] = k;
+      }
+    } else {
+      for (uint32_t j = threadIdx.x; j < count; j += kRsThreads) {
+        const K k = buf[j];
+        out[gofs[(uint32_t)(k >> shift) & mask] + j] = k;
+      }
     }
-    __syncthreads();
   }
 }
 
-template <typename K>
-static void launch_scatter(const Launch& L, int nb, int w, const K* in, K* out, uint64_t n,
-                           uint64_t chunk, int shift, const uint32_t* offs,
-                           const uint32_t* digit_tot, const uint64_t* d_n) {
-#define SRDL_SCATTER_CASE(DB)                                                          \
-  case DB:                                                                             \
-    prefer_shared(rs_scatter<K, DB>);                                                  \
-    rs_scatter<K, DB><<<nb, kRsThreads, 0, L.stream>>>(in, out, n, chunk, shift, offs, \
-                                                       digit_tot, d_n);                \
-    break;
+// Lets a scatter kernel use its shared memory on the current device.
+template <typename K, int DB, bool FIRST>
+static void allow_scatter() {
+  static std::atomic<uint64_t> done{0};  // devices the attributes are set on
+  int dev = 0;
+  SRDL_CUDA(cudaGetDevice(&dev));
+  const uint64_t bit = 1ull << (dev & 63);
+  if (done.load(std::memory_order_acquire) & bit) return;
+  SRDL_CUDA(cudaFuncSetAttribute(rs_scatter<K, DB, FIRST>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 (int)cudaSharedmemCarveoutMaxShared));
+  SRDL_CUDA(cudaFuncSetAttribute(rs_scatter<K, DB, FIRST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)rs_smem_bytes<K, DB>()));
+  done.fetch_or(bit, std::memory_order_release);
+}
+
+// f(std::integral_constant<int, w>) for the digit width w.
+template <typename K, typename F>
+static void with_digit(int w, F&& f) {
+#define SRDL_DIGIT_CASE(DB)                    \
+  case DB:                                     \
+    f(std::integral_constant<int, DB>{});      \
+    return;
   switch (w) {
-    SRDL_SCATTER_CASE(1)
-    SRDL_SCATTER_CASE(2)
-    SRDL_SCATTER_CASE(3)
-    SRDL_SCATTER_CASE(4)
-    SRDL_SCATTER_CASE(5)
-    SRDL_SCATTER_CASE(6)
-    SRDL_SCATTER_CASE(7)
-    SRDL_SCATTER_CASE(8)
+    SRDL_DIGIT_CASE(1)
+    SRDL_DIGIT_CASE(2)
+    SRDL_DIGIT_CASE(3)
+    SRDL_DIGIT_CASE(4)
+    SRDL_DIGIT_CASE(5)
+    SRDL_DIGIT_CASE(6)
+    SRDL_DIGIT_CASE(7)
+    SRDL_DIGIT_CASE(8)
+    SRDL_DIGIT_CASE(9)
     default:
       throw Error{kErrState, "radix sort: digit width out of range"};
   }
-#undef SRDL_SCATTER_CASE
+#undef SRDL_DIGIT_CASE
+}
+
+// One counting pass: histogram, offsets, scatter.
+template <typename K, bool FIRST>
+static void radix_pass(const Launch& L, int nb, int w, const void* in, K* out, uint64_t n, uint64_t chunk, int shift,
+                       uint32_t* counts, uint32_t* digit_tot, const uint64_t* d_n, int bits, bool swap) {
+  rs_hist<K, FIRST><<<nb, kRsThreads, 0, L.stream>>>(in, n, chunk, shift, 1 << w, counts, d_n, bits, swap);
+  rs_rowscan<<<1 << w, kRsScanThreads, 0, L.stream>>>(counts, nb, digit_tot);
+  with_digit<K>(w, [&](auto db) {
+    constexpr int DB = decltype(db)::value;
+    allow_scatter<K, DB, FIRST>();
+    rs_scatter<K, DB, FIRST><<<nb, kRsThreads, rs_smem_bytes<K, DB>(), L.stream>>>(
+        in, out, n, chunk, shift, counts, digit_tot, d_n, bits, swap);
+  });
+  SRDL_CUDA(cudaGetLastError());
+  count_launches(3);
+}
+
+int radix_passes(const Launch& L, int dom_bits) {
+  const int maxw = L.radix_bits >= 1 && L.radix_bits <= 7 ? L.radix_bits : kRsAutoBits;
+  return (2 * dom_bits + maxw - 1) / maxw;
 }
 
 static inline bool use32(int bits) { return 2 * bits <= 32; }
@@ -295,7 +411,7 @@ size_t sort_dev_scratch_bytes(uint64_t cap, uint64_t full_cap, int bits) {
 
 size_t sort_scratch_bytes(uint64_t n, int bits) {
   const size_t ks = use32(bits) ? 4 : 8;
-  const size_t counts = (size_t)kRsBins * 256 * 8 * 4;  // <= 8 blocks per SM, 256 SMs
+  const size_t counts = (size_t)256 * 256 * 8 * 4;  // 2^9 digits of 4 blocks, or 2^10 of 2, on each of 256 SMs
   return 2 * (((n * ks) + 255) & ~size_t(255)) + counts + 2048 + cp_scratch_bytes(n) + 1024;
 }
 
@@ -308,34 +424,22 @@ static void sort_dedup_t(const Launch& L, const uint64_t* in, uint64_t n, int bi
   SRDL_REQUIRE(n < (1ull << 32), kErrCapacity, "sort: more than 2^32-1 rows in one index");
   K* a = s.take<K>(n);
   K* b = s.take<K>(n);
-  const int pgrid = (int)std::min<uint64_t>((n + 255) / 256, (uint64_t)L.num_sms * 16);
-  rs_pack<K><<<pgrid ? pgrid : 1, 256, 0, L.stream>>>(in, n, bits, swap, a, d_n);
-  SRDL_CUDA(cudaGetLastError());
-  count_launches(1);
-
-  // Tile partition shared by the histogram and scatter launches (with the
-  // count on the device, the blocks derive the same even split from it).
-  const uint64_t tiles = (n + kRsTile - 1) / kRsTile;
-  const uint64_t cap = (uint64_t)L.num_sms * 8;
-  const uint64_t per = (tiles + cap - 1) / cap;
-  const uint64_t chunk = (per ? per : 1) * kRsTile;
-  const int nb = (int)((n + chunk - 1) / chunk);
-  const uint64_t kchunk = d_n ? 0 : chunk;
-  uint32_t* counts = s.take<uint32_t>((size_t)kRsBins * nb);
-  uint32_t* digit_tot = s.take<uint32_t>(kRsBins);
-
+  // Even split of the keys over the resident blocks, shared by the histogram
+  // and scatter launches (with the count on the device, the blocks derive the
+  // same split from it).
+  const uint64_t resident = (uint64_t)L.num_sms * kRsBlocksPerSm;
+  const int nb = (int)std::min<uint64_t>(resident, (n + kRsMinChunk - 1) / kRsMinChunk);
+  const uint64_t chunk = rs_chunk(n, nb);
   const int total_bits = 2 * bits;
-  const int maxw = L.radix_bits >= 1 && L.radix_bits <= 8 ? L.radix_bits : 8;
-  const int passes = (total_bits + maxw - 1) / maxw;
+  const int passes = radix_passes(L, bits);
+  uint32_t* counts = s.take<uint32_t>((size_t)nb << ((total_bits + passes - 1) / passes));
+  uint32_t* digit_tot = s.take<uint32_t>((size_t)1 << kRsMaxBits);
+
   int shift = 0;
-  for (int p = 0; p < passes && (n > 1 || d_n); p++) {
+  for (int p = 0; p < passes; p++) {
     const int w = total_bits / passes + (p < total_bits % passes ? 1 : 0);
-    const int nbins = 1 << w;
-    rs_hist<K><<<nb, kRsThreads, 0, L.stream>>>(a, n, kchunk, shift, nbins, counts, d_n);
-    rs_rowscan<<<nbins, kRsThreads, 0, L.stream>>>(counts, nb, digit_tot);
-    launch_scatter<K>(L, nb, w, a, b, n, kchunk, shift, counts, digit_tot, d_n);
-    SRDL_CUDA(cudaGetLastError());
-    count_launches(3);
+    if (p == 0) radix_pass<K, true>(L, nb, w, in, b, n, chunk, shift, counts, digit_tot, d_n, bits, swap);
+    else radix_pass<K, false>(L, nb, w, a, b, n, chunk, shift, counts, digit_tot, d_n, bits, swap);
     std::swap(a, b);
     shift += w;
   }
@@ -363,14 +467,11 @@ void sort_dedup(const Launch& L, const uint64_t* in, uint64_t n, int bits, bool 
 
 template <typename K>
 static void warm_sort_kernels() {
-  prefer_shared(rs_scatter<K, 1>);
-  prefer_shared(rs_scatter<K, 2>);
-  prefer_shared(rs_scatter<K, 3>);
-  prefer_shared(rs_scatter<K, 4>);
-  prefer_shared(rs_scatter<K, 5>);
-  prefer_shared(rs_scatter<K, 6>);
-  prefer_shared(rs_scatter<K, 7>);
-  prefer_shared(rs_scatter<K, 8>);
+  for (int w = 1; w <= kRsMaxBits; w++)
+    with_digit<K>(w, [](auto db) {
+      allow_scatter<K, decltype(db)::value, true>();
+      allow_scatter<K, decltype(db)::value, false>();
+    });
 }
 
 void warm_device_loop_kernels(int bits) {

@@ -8,12 +8,25 @@ import pytest
 from conftest import load_plan
 from srdatalog_b200 import native
 from srdatalog_b200 import workloads as W
-from test_gpu_primitives import gpu_diff, gpu_merge, keys_with_bits
+from test_gpu_primitives import gpu_diff, gpu_merge, gpu_sort_unique, keys_with_bits
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip('torch')
 
 TOP = np.uint64(0xFFFFFFFFFFFFFFFF)
+
+
+@pytest.mark.parametrize('n', [5000, 300_000])
+def test_sort_unique_one_digit(n):
+  '''Every key equal, then all but one (largest counters of a tile, keys of all ones).'''
+  k = np.full(n, TOP, np.uint64)
+  assert np.array_equal(gpu_sort_unique(k, 32), np.array([TOP]))
+  k[n // 3] = 0
+  assert np.array_equal(gpu_sort_unique(k, 32), np.array([0, TOP], np.uint64))
+  k16 = np.full(n, (0xFFFF << 32) | 0xFFFF, np.uint64)   # all ones in 32-bit packed form
+  assert np.array_equal(gpu_sort_unique(k16, 16), k16[:1])
+  assert np.array_equal(gpu_sort_unique(np.sort(keys_with_bits(np.random.default_rng(n), n, 7)), 7),
+                        oracle.sort_unique(keys_with_bits(np.random.default_rng(n), n, 7)))
 
 
 @pytest.mark.parametrize('na,nb', [(1, 4), (2047, 2049), (2048, 2048), (31, 6000), (4096, 4096 * 16),
