@@ -344,6 +344,145 @@ __global__ void __launch_bounds__(kRsThreads, 2) rs_scatter(const void* __restri
   }
 }
 
+// ---- at most kRsSmall keys: one block, one launch ----------------------------
+//
+// A small request's or a late iteration's tuples cost launches, not work: the
+// passes above take three launches each whatever the count, about 3 us apiece.
+// One block holds up to 16384 keys in shared memory, runs every counting pass
+// there (8-bit digits, ranked by rs_rank), drops repeats and the keys
+// found in FULL or HEAD (one interleaved binary search per key) and writes the
+// rest in order.  Bound: one SM's issue slots; 5000 keys of 34 bits take 46 us
+// with the count read back (109 us in 16 launches), 16,000 keys 71 us (95 us).
+constexpr int kRsSmallThreads = 1024;
+constexpr int kRsSmallWarps = kRsSmallThreads / 32;
+constexpr uint64_t kRsSmall = (uint64_t)kRsSmallThreads * kRsItems;
+constexpr int kRsSmallBits = 8;
+constexpr int kRsSmallPairs = 1 << (kRsSmallBits - 1);
+
+template <typename K>
+constexpr size_t rs_small_smem_bytes() {
+  return kRsSmall * sizeof(K) + (size_t)kRsSmallWarps * kRsSmallPairs * 4;
+}
+
+template <typename K>
+__global__ void __launch_bounds__(kRsSmallThreads, 1) rs_small_kernel(const uint64_t* in, uint32_t n, int bits,
+                                                                      bool swap, int passes, DedupDiffSel<K> sel,
+                                                                      uint64_t* d_nout) {
+  extern __shared__ __align__(16) unsigned char rs_sm[];
+  K* buf = reinterpret_cast<K*>(rs_sm);
+  uint32_t* cnt = reinterpret_cast<uint32_t*>(rs_sm + kRsSmall * sizeof(K));
+  __shared__ uint32_t scan_sh[kRsSmallWarps + 1];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const unsigned lt = lanemask_lt(), gt = ~(lt | (1u << lane));
+  const int rounds = (int)((n + kRsSmallThreads - 1) / kRsSmallThreads);
+  const uint32_t i0 = (uint32_t)(wid * rounds * 32 + lane);  // this lane's keys: i0, i0 + 32, ...
+  uint32_t* my = cnt + wid * kRsSmallPairs;
+  uint16_t* my16 = reinterpret_cast<uint16_t*>(my);
+  K key[kRsItems];
+#pragma unroll
+  for (int r = 0; r < kRsItems; r++) {
+    key[r] = ~K(0);  // behind every real key, in every pass
+    if (r < rounds && i0 + r * 32 < n) key[r] = rs_packed<K>(in[i0 + r * 32], bits, swap);
+  }
+  const int total = 2 * bits;
+  int shift = 0;
+  for (int p = 0; p < passes; p++) {
+    const int w = total / passes + (p < total % passes ? 1 : 0);
+    const uint32_t mask = (1u << w) - 1;
+    for (int i = lane; i < kRsSmallPairs; i += 32) my[i] = 0;
+    __syncwarp();
+    uint32_t rank[kRsItems / 2];
+#pragma unroll
+    for (int r = 0; r < kRsItems; r++) {
+      if (r < rounds) {
+        const uint32_t rk = rs_rank<kRsSmallBits>(my16, (uint32_t)(key[r] >> shift) & mask, lt, gt);
+        rank[r / 2] = r & 1 ? rank[r / 2] | (rk << 16) : rk;
+      }
+    }
+    __syncthreads();
+    {
+      const int t = threadIdx.x;
+      uint32_t run = 0;
+      if (t < kRsSmallPairs) {
+#pragma unroll 8
+        for (int q = 0; q < kRsSmallWarps; q++) {
+          const uint32_t v = cnt[q * kRsSmallPairs + t];
+          cnt[q * kRsSmallPairs + t] = run;
+          run += v;
+        }
+      }
+      const uint32_t c0 = run & 0xffffu, c1 = run >> 16;
+      uint32_t all;
+      const uint32_t start = block_excl_scan(c0 + c1, scan_sh, &all);
+      if (t < kRsSmallPairs) {
+        const uint32_t add = start | ((start + c0) << 16);
+#pragma unroll 8
+        for (int q = 0; q < kRsSmallWarps; q++) cnt[q * kRsSmallPairs + t] += add;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kRsItems; r++) {
+      if (r < rounds) {
+        const uint32_t rk = r & 1 ? rank[r / 2] >> 16 : rank[r / 2] & 0xffffu;
+        buf[my16[(uint32_t)(key[r] >> shift) & mask] + rk] = key[r];
+      }
+    }
+    __syncthreads();
+    if (p + 1 < passes) {
+#pragma unroll
+      for (int r = 0; r < kRsItems; r++)
+        if (r < rounds) key[r] = buf[i0 + r * 32];
+    }
+    shift += w;
+  }
+  // sorted: keep the first of equal keys that FULL and HEAD do not have
+  uint32_t kept = 0, found = 0;  // bit r: this lane's key of round r; the warp's count
+#pragma unroll
+  for (int g = 0; g < kRsItems; g += kDdKeys) {
+    if (g < rounds) {
+      uint64_t k[kDdKeys];
+      bool keep[kDdKeys], hit[kDdKeys];
+#pragma unroll
+      for (int q = 0; q < kDdKeys; q++) {
+        const uint32_t i = i0 + (g + q) * 32;
+        const K c = g + q < rounds ? buf[i] : K(0);
+        keep[q] = g + q < rounds && i < n && (i == 0 || buf[i - 1] != c);
+        k[q] = sel.expand(c);
+      }
+      if (sel.n_full) {
+        dd_lower_bounds(sel.full, sel.n_full, k, hit);
+#pragma unroll
+        for (int q = 0; q < kDdKeys; q++) keep[q] &= !hit[q];
+      }
+      if (sel.n_head) {
+        dd_lower_bounds(sel.head, sel.n_head, k, hit);
+#pragma unroll
+        for (int q = 0; q < kDdKeys; q++) keep[q] &= !hit[q];
+      }
+#pragma unroll
+      for (int q = 0; q < kDdKeys; q++) {
+        kept |= (keep[q] ? 1u : 0u) << (g + q);
+        found += __popc(__ballot_sync(kAllLanes, keep[q]));
+      }
+    }
+  }
+  uint32_t tot;
+  // (lane 0 carries the warp's count, so the warp's first position is its prefix)
+  uint32_t pos = block_excl_scan(lane == 0 ? found : 0u, scan_sh, &tot);
+  pos = __shfl_sync(kAllLanes, pos, 0);
+#pragma unroll
+  for (int r = 0; r < kRsItems; r++) {
+    if (r < rounds) {
+      const bool f = (kept >> r) & 1u;
+      const unsigned m = __ballot_sync(kAllLanes, f);
+      if (f) sel.store(pos + __popc(m & lt), sel.expand(buf[i0 + r * 32]));
+      pos += __popc(m);
+    }
+  }
+  if (threadIdx.x == 0) *d_nout = tot;
+}
+
 // Lets a scatter kernel use its shared memory on the current device.
 template <typename K, int DB, bool FIRST>
 static void allow_scatter() {
@@ -357,6 +496,25 @@ static void allow_scatter() {
   SRDL_CUDA(cudaFuncSetAttribute(rs_scatter<K, DB, FIRST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)rs_smem_bytes<K, DB>()));
   done.fetch_or(bit, std::memory_order_release);
+}
+
+template <typename K>
+static void sort_small(const Launch& L, const uint64_t* in, uint64_t n, int bits, bool swap,
+                       const DedupDiffSel<K>& sel, uint64_t* d_nout) {
+  static std::atomic<uint64_t> done{0};  // devices the attribute is set on
+  int dev = 0;
+  SRDL_CUDA(cudaGetDevice(&dev));
+  const uint64_t bit = 1ull << (dev & 63);
+  if (!(done.load(std::memory_order_acquire) & bit)) {
+    SRDL_CUDA(cudaFuncSetAttribute(rs_small_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)rs_small_smem_bytes<K>()));
+    done.fetch_or(bit, std::memory_order_release);
+  }
+  const int passes = (2 * bits + kRsSmallBits - 1) / kRsSmallBits;
+  rs_small_kernel<K><<<1, kRsSmallThreads, rs_small_smem_bytes<K>(), L.stream>>>(in, (uint32_t)n, bits, swap, passes,
+                                                                                sel, d_nout);
+  SRDL_CUDA(cudaGetLastError());
+  count_launches(1);
 }
 
 // f(std::integral_constant<int, w>) for the digit width w.
@@ -424,6 +582,11 @@ static void sort_dedup_t(const Launch& L, const uint64_t* in, uint64_t n, int bi
   SRDL_REQUIRE(n < (1ull << 32), kErrCapacity, "sort: more than 2^32-1 rows in one index");
   K* a = s.take<K>(n);
   K* b = s.take<K>(n);
+  if (!d_n && n <= kRsSmall) {
+    DedupDiffSel<K> sel{nullptr, bits, true, full, full ? n_full : 0, out, head, head ? n_head : 0};
+    sort_small<K>(L, in, n, bits, swap, sel, d_nout);
+    return;
+  }
   // Even split of the keys over the resident blocks, shared by the histogram
   // and scatter launches (with the count on the device, the blocks derive the
   // same split from it).

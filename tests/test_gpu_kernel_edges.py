@@ -16,6 +16,16 @@ torch = pytest.importorskip('torch')
 TOP = np.uint64(0xFFFFFFFFFFFFFFFF)
 
 
+# one block sorts up to 16,384 keys; above, blocks take at least 2,048 keys and
+# tiles of at most 8,192; digits are 5 to 9 bits wide
+@pytest.mark.parametrize('bits', [2, 13, 16, 19, 32])
+@pytest.mark.parametrize('n', [2, 1023, 1025, 16_383, 16_384, 16_385, 40_961, 2_424_833])
+def test_sort_unique_block_edges(n, bits):
+  rng = np.random.default_rng(n + bits)
+  k = keys_with_bits(rng, n, bits, dup_frac=0.2)
+  assert np.array_equal(gpu_sort_unique(k, bits), oracle.sort_unique(k))
+
+
 @pytest.mark.parametrize('n', [5000, 300_000])
 def test_sort_unique_one_digit(n):
   '''Every key equal, then all but one (largest counters of a tile, keys of all ones).'''
