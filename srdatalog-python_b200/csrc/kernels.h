@@ -178,6 +178,10 @@ void split3(const Launch& L, const uint64_t* keys, uint64_t n, int bits, int hal
 // Swap the two 32-bit halves of every key (index permutation (1,0) <-> (0,1)).
 void swap_halves(const Launch& L, const uint64_t* in, uint64_t n, uint64_t* out);
 
+// Row-major uint32 rows of arity 1 or 2 from keys in declared column order;
+// `out` (16-byte aligned) may be page-locked host memory.
+void unpack_rows(const Launch& L, const uint64_t* keys, uint64_t n, int arity, void* out);
+
 // Exclusive scan of n uint64 values; out has n+1 entries (out[n] = total, also
 // written to *total when given).
 size_t scan_scratch_bytes(uint64_t n);

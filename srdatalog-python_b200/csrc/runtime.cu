@@ -15,7 +15,6 @@ namespace srdl {
 // Dense directories are built while the value domain stays below this many
 // entries (64 MB of uint32 offsets); above it, lookups binary-search keys.
 constexpr uint64_t kDenseDirMax = 1ull << 24;
-constexpr int kSmallSlots = 16;
 
 static thread_local std::string g_last_error;
 void set_error(const std::string& msg) { g_last_error = msg; }
@@ -250,6 +249,24 @@ void DevBuf::reset() {
   bytes_ = 0;
 }
 
+void PinnedBuf::reserve(size_t bytes) {
+  if (bytes <= cap) return;
+  release();
+  SRDL_CUDA(cudaMallocHost(&p, bytes));
+  cap = bytes;
+}
+
+void PinnedBuf::release() {
+  if (p) (void)cudaFreeHost(p);
+  p = nullptr;
+  cap = 0;
+}
+
+DumpStage& dump_stage() {
+  static auto* s = new DumpStage();
+  return *s;
+}
+
 // ------------------------------------------------------------------ plan
 
 static Ver parse_ver(const std::string& s) {
@@ -288,6 +305,11 @@ Database::~Database() {
     arena_detach(L_.stream);
     cudaStreamSynchronize(L_.stream);
     if (h_small_) cudaFreeHost(h_small_);
+    dump_buf_.release();
+    if (--dump_stage().users == 0) {
+      std::lock_guard<std::mutex> g(dump_stage().mu);
+      if (dump_stage().users == 0) dump_stage().buf.release();
+    }
     for (auto& kv : rels_)
       if (kv.second->pinned) cudaFreeHost(kv.second->pinned);
     for (auto& e : kev_) {
@@ -479,8 +501,9 @@ void Database::init_device() {
   uint64_t thr = ~0ull;
   SRDL_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr));
   arena_attach(L_.stream);
-  SRDL_CUDA(cudaMallocHost(&h_small_, kSmallSlots * sizeof(uint64_t)));
+  SRDL_CUDA(cudaMallocHost(&h_small_, kSmallSlots * sizeof(uint64_t) + kSmallRows));
   d_small_ = DevBuf(kSmallSlots * sizeof(uint64_t), L_.stream);
+  dump_stage().users++;
   dev_ready_ = true;
 }
 

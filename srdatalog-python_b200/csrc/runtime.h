@@ -6,10 +6,12 @@
 // The plan is interpreted; kernels are fixed.
 #pragma once
 
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -20,6 +22,28 @@
 namespace srdl {
 
 enum Ver { kFull = 0, kDelta = 1, kNew = 2 };
+
+constexpr int kSmallSlots = 16;           // scalars the host reads back
+constexpr size_t kSmallRows = 64 << 10;   // bytes of rows read back through the same page-locked block
+constexpr int kDumpThreads = 8;           // larger results: host threads, and
+constexpr uint64_t kDumpPiece = 2 << 20;  // bytes of rows a thread moves at a time
+
+// Page-locked host memory that grows on demand.
+struct PinnedBuf {
+  void* p = nullptr;
+  size_t cap = 0;
+  void reserve(size_t bytes);
+  void release();
+};
+
+// The process's page-locked pieces for reading large results back, freed with
+// the last initialised database.
+struct DumpStage {
+  std::mutex mu;  // held by the handle that uses buf
+  PinnedBuf buf;
+  std::atomic<int> users{0};
+};
+DumpStage& dump_stage();
 
 // Caching arena for the allocations of one stream.  Freed blocks are kept in
 // per-size-class free lists and handed to the next allocation of that class
@@ -380,13 +404,15 @@ class Database {
   void prof_end(size_t id, double bytes, double units);
   void prof_collect();
   DevBuf d_small_;  // device scalars read back by the host
-  uint64_t* h_small_ = nullptr;  // pinned mirror
+  uint64_t* h_small_ = nullptr;  // pinned mirror, and kSmallRows bytes for small results
+  PinnedBuf dump_buf_;           // larger results, when the process's pieces are taken (copy_rows)
 
   // ------------------------------------------------------------ helpers
   void parse_plan(const std::string& plan_json);
   void reset_device_state();
   void upload_inputs();
   uint64_t read_scalar(int slot);
+  void copy_rows(const uint64_t* keys, uint64_t n, int arity, uint32_t* out);
   Index& ensure_index(Relation& r, Ver v, const std::vector<int>& perm);
   // FULL's large segment in `perm` without merging HEAD into it.
   Index& full_base(Relation& r, const std::vector<int>& perm);

@@ -266,6 +266,42 @@ void swap_halves(const Launch& L, const uint64_t* in, uint64_t n, uint64_t* out)
   count_launches(1);
 }
 
+// A row (c0, c1) is the key with its halves swapped: rows pass through as
+// 16-byte stores of two rows (four unary ones), which cross PCIe in full lines.
+__global__ void unpack_rows_kernel(const uint64_t* __restrict__ keys, uint64_t n, int arity,
+                                   uint32_t* __restrict__ out) {
+  const uint64_t step = (uint64_t)gridDim.x * blockDim.x, first = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  if (arity == 2) {
+    for (uint64_t i = first; i < n / 2; i += step) {
+      const uint64_t k0 = keys[2 * i], k1 = keys[2 * i + 1];
+      reinterpret_cast<uint4*>(out)[i] =
+          make_uint4((uint32_t)(k0 >> 32), (uint32_t)k0, (uint32_t)(k1 >> 32), (uint32_t)k1);
+    }
+    if (first == 0 && (n & 1)) {
+      out[2 * n - 2] = (uint32_t)(keys[n - 1] >> 32);
+      out[2 * n - 1] = (uint32_t)keys[n - 1];
+    }
+  } else {
+    for (uint64_t i = first; i < n / 4; i += step) {
+      uint4 v;
+      v.x = (uint32_t)(keys[4 * i] >> 32);
+      v.y = (uint32_t)(keys[4 * i + 1] >> 32);
+      v.z = (uint32_t)(keys[4 * i + 2] >> 32);
+      v.w = (uint32_t)(keys[4 * i + 3] >> 32);
+      reinterpret_cast<uint4*>(out)[i] = v;
+    }
+    if (first < (n & 3)) out[(n & ~uint64_t(3)) + first] = (uint32_t)(keys[(n & ~uint64_t(3)) + first] >> 32);
+  }
+}
+
+void unpack_rows(const Launch& L, const uint64_t* keys, uint64_t n, int arity, void* out) {
+  if (!n) return;
+  unpack_rows_kernel<<<grid_for((n + 1) / 2, L.num_sms), 256, 0, L.stream>>>(keys, n, arity,
+                                                                           static_cast<uint32_t*>(out));
+  SRDL_CUDA(cudaGetLastError());
+  count_launches(1);
+}
+
 // ---- ternary relations: column orders and the pair / row views ---------------
 // A ternary tuple (x0, x1, x2) in some column order is one uint64 key: P =
 // x0 << 2b | x1 << b | x2, stored split at `half` bits as

@@ -63,6 +63,20 @@ def test_merge_tile_edges(na, nb, apart):
   assert np.array_equal(gpu_merge(a, b), oracle.merge(a, b))
 
 
+@pytest.mark.parametrize('n', [8191, 8192, 8193, 262_144, 262_145, 2_400_007])
+def test_dump_piece_edges(n):
+  '''Results read back in one small piece, in one large one and in several.'''
+  rng = np.random.default_rng(n)
+  k = np.unique(keys_with_bits(rng, n + n // 8 + 64, 20))
+  k = rng.permutation(k)[:n]
+  rows = np.stack([k >> np.uint64(32), k & np.uint64(0xFFFFFFFF)], 1).astype(np.uint32)
+  with native.Database(load_plan('triangle')) as db:
+    db.load_rows('KnowsInput', rows)
+    db.run()
+    for _ in range(2):
+      assert np.array_equal(db.dump('Knows'), rows[np.argsort(k)])
+
+
 @pytest.mark.parametrize('m', [4095, 4096, 4097, 16_384, 16_385, 120_000])
 def test_count_scan_edges(m):
   '''Tables on both sides of the one-block count and scan.'''
