@@ -342,8 +342,15 @@ __device__ __forceinline__ uint64_t dev_warp_chunk(const JoinDev& jd, uint64_t c
   return (((total + warps - 1) / warps) + 31) & ~uint64_t(31);
 }
 
+// Adds a key to the bitmap set a launch emits into (JoinDev::set_words).
+__device__ __forceinline__ void set_key(const JoinDev& jd, uint64_t key) {
+  const uint32_t p = ((uint32_t)(key >> 32) << jd.set_bits) | (uint32_t)key;
+  atomicOr(jd.set_words + (p >> 5), 1u << (p & 31));
+}
+
 // Warp-aggregated append of the m-set lanes' keys at *d_out_n; with an
-// output capacity, positions past it are dropped and raise the flag.
+// output capacity, positions past it are dropped and raise the flag.  Keys
+// that go to a set are only counted there.
 __device__ __forceinline__ void append_key(const JoinDev& jd, unsigned m, bool ok, int lane,
                                            unsigned long long* d_out_n, uint64_t* out_keys,
                                            uint64_t key) {
@@ -351,6 +358,10 @@ __device__ __forceinline__ void append_key(const JoinDev& jd, unsigned m, bool o
   const int leader = __ffs(m) - 1;
   unsigned long long pos0 = 0;
   if (lane == leader) pos0 = atomicAdd(d_out_n, (unsigned long long)__popc(m));
+  if (jd.set_words) {
+    if (ok) set_key(jd, key);
+    return;
+  }
   pos0 = __shfl_sync(kAllLanes, pos0, leader);
   const uint64_t pos = pos0 + __popc(m & lanemask_lt());
   if (jd.out_cap && pos0 + __popc(m) > jd.out_cap && lane == leader && jd.d_overflow)
@@ -788,7 +799,9 @@ __global__ void __launch_bounds__(kJThreads) join_cart2_kernel(
             const int ks = lv.key_slot[i];
             kc[i] = i >= lv.key_arity ? 0u : ks == s0 ? v0 : ks == s1 ? v1 : slot_value(in, ks, r);
           }
-          if (!jd.out_cap || base + lane < jd.out_cap) out_keys[base + lane] = emit_key(lv, kc);
+          const uint64_t key = emit_key(lv, kc);
+          if (jd.set_words) set_key(jd, key);
+          else if (!jd.out_cap || base + lane < jd.out_cap) out_keys[base + lane] = key;
         }
         r0 = __shfl_sync(kAllLanes, r, 31);
         continue;

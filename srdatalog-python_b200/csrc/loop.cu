@@ -22,7 +22,14 @@
 // the conditions: the loop stops on an empty delta (the fixpoint), at the
 // run's iteration limit, or when a kernel found a capacity too small (the
 // overflow flag; kernels never write past a capacity).  One launch, one
-// host synchronisation.  On overflow the failed iteration's inputs are
+// host synchronisation.
+//
+// Where the key space is small (2^kKeysetMaxBits), NEW and FULL are bitmap sets
+// during the loop: the joins set the bits of the keys they derive, those FULL
+// lacks are listed as DELTA and added to FULL, and FULL is listed as a sorted
+// array once, after the last iteration -- no rule of a qualifying step reads it
+// before.  That takes the place of the sort, the set difference and the merge
+// of every iteration.  On overflow the failed iteration's inputs are
 // intact (they are the other buffer set): the host resumes from them on the
 // host path, and the next entry sizes the buffers from the larger counts
 // that path measures.  Results are those of the host path: the same
@@ -58,8 +65,9 @@ struct LoopCtl {
 };
 
 // ks: packed key bytes of the sort, passes: its counting passes.
+// (ks 0: bitmap sets of set_bytes each)
 __global__ void loop_ctrl_kernel(LoopCtl* ctl, LoopCounts* cnt, int nrel, int p, int ks, int passes,
-                                 cudaGraphConditionalHandle hw, cudaGraphConditionalHandle hi,
+                                 double set_bytes, cudaGraphConditionalHandle hw, cudaGraphConditionalHandle hi,
                                  int set_if) {
   if (blockIdx.x != 0 || threadIdx.x != 0) return;
   ctl->bodies++;
@@ -75,8 +83,11 @@ __global__ void loop_ctrl_kernel(LoopCtl* ctl, LoopCounts* cnt, int nrel, int p,
       cnt[r].derived += cnt[r].n_new;
       // emitted keys, the sort with its fused difference, the merge and
       // the delta's trie view -- the bytes the host path charges for them
-      ctl->alg_bytes += 8.0 * nn + passes * 2.0 * ks * nn + 8.0 * nn + 2.0 * ks * nn + 8.0 * nd +
-                        8.0 * nn + 16.0 * (nf + nd) + 16.0 * nd;
+      if (ks)
+        ctl->alg_bytes += 8.0 * nn + passes * 2.0 * ks * nn + 8.0 * nn + 2.0 * ks * nn + 8.0 * nd +
+                          8.0 * nn + 16.0 * (nf + nd) + 16.0 * nd;
+      else
+        ctl->alg_bytes += 8.0 * nn + 2.0 * set_bytes + 8.0 * nd + 16.0 * nd;
     }
     go = delta > 0 && ctl->done < ctl->remaining;
   }
@@ -104,6 +115,7 @@ struct LoopRel {
   int producers = 0;  // execute ops inserting into it
   DevBuf newk, sort_scr, trie_scr;
   DevBuf full[2], delta[2], lo[2], roots[2], dir[2];
+  DevBuf new_set, full_set, set_counts;  // bitmap sets: in place of sort_scr and full[]
 };
 
 // Buffers of one join level of one pipeline.
@@ -219,6 +231,14 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
 
   LoopCtx X;
   X.dir_n = dom_max_ + 2;
+  // Bitmap sets for NEW and FULL: always up to 2^26 keys, whose 8 MB an iteration
+  // goes over in less time than the launches they replace take; above when an
+  // iteration has been seen to fill them as a sort would have to.  Not under a
+  // memory limit, whose runs keep the footprint they had.
+  bool sets = 2 * bits_ <= std::min(kKeysetMaxBits, 26);
+  for (auto& name : comp) sets = sets || sort_by_keyset(new_max_[name], bits_);
+  sets = sets && !opt_mem_limit_;
+  const size_t set_bytes = sets ? keyset_words(bits_) * 4 : 0;
   // ---- capacities and buffers (an allocation refused by the run's memory
   //      limit leaves the step to the host path)
   try {
@@ -251,8 +271,10 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
       {
         // the buffers below; leave the step to the host path rather than
         // take most of the free memory (the host path needs far less)
-        const uint64_t need = lr.cap_new * 8 + lr.cap_delta * (16 + 8 + 8) +
-                              sort_dev_scratch_bytes(lr.cap_new, lr.cap_full, bits_) + lr.cap_full * 16;
+        const uint64_t need = lr.cap_delta * (16 + 8 + 8) +
+                              (sets ? 2 * set_bytes
+                                    : lr.cap_new * 8 + lr.cap_full * 16 +
+                                          sort_dev_scratch_bytes(lr.cap_new, lr.cap_full, bits_));
         size_t free_b = 0, total_b = 0;
         SRDL_CUDA(cudaMemGetInfo(&free_b, &total_b));
         const ArenaUse au = arena_use(L_.stream);
@@ -260,11 +282,17 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
           throw Error{kErrCapacity, "device loop buffers (" + std::to_string(need >> 20) +
                                         " MB) would take most of the free device memory"};
       }
-      lr.newk = DevBuf(lr.cap_new * 8, L_.stream);
-      lr.sort_scr = DevBuf(sort_dev_scratch_bytes(lr.cap_new, lr.cap_full, bits_), L_.stream);
+      if (!sets) lr.newk = DevBuf(lr.cap_new * 8, L_.stream);
+      if (sets) {
+        lr.new_set = DevBuf(set_bytes, L_.stream);
+        lr.full_set = DevBuf(set_bytes, L_.stream);
+        lr.set_counts = DevBuf(keyset_counts(L_, bits_) * 4, L_.stream);
+      } else {
+        lr.sort_scr = DevBuf(sort_dev_scratch_bytes(lr.cap_new, lr.cap_full, bits_), L_.stream);
+      }
       lr.trie_scr = DevBuf(trie_scratch_bytes(lr.cap_delta) + 1024, L_.stream);
       for (int q = 0; q < 2; q++) {
-        lr.full[q] = DevBuf(lr.cap_full * 8, L_.stream);
+        if (!sets) lr.full[q] = DevBuf(lr.cap_full * 8, L_.stream);
         lr.delta[q] = DevBuf(lr.cap_delta * 8, L_.stream);
         lr.lo[q] = DevBuf(lr.cap_delta * 4, L_.stream);
         lr.roots[q] = DevBuf(lr.cap_delta * 4, L_.stream);
@@ -320,9 +348,13 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
     auto dit = r.v[kDelta].idx.find(r.canonical);
     const uint64_t dn = dit == r.v[kDelta].idx.end() ? 0 : dit->second.n;
     LoopCounts* c = X.cnt_d() + i;
-    if (f.n)
+    if (sets) {
+      keyset_from_sorted(L_, f.keys.as<uint64_t>(), f.n, bits_, lr.full_set.as<uint32_t>());
+      SRDL_CUDA(cudaMemsetAsync(lr.new_set.as<void>(), 0, set_bytes, L_.stream));
+    } else if (f.n) {
       SRDL_CUDA(cudaMemcpyAsync(lr.full[0].as<void>(), f.keys.as<void>(), f.n * 8, cudaMemcpyDeviceToDevice,
                                 L_.stream));
+    }
     if (dn)
       SRDL_CUDA(cudaMemcpyAsync(lr.delta[0].as<void>(), dit->second.keys.as<void>(), dn * 8,
                                 cudaMemcpyDeviceToDevice, L_.stream));
@@ -421,8 +453,10 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
           lv.emit = kEmitKeys;
           lv.key_arity = 2;
           for (int c = 0; c < 2; c++) lv.key_slot[c] = pp.key_slot[c];
-          jd.out_cap = lr.cap_new;
+          jd.out_cap = sets ? 0 : lr.cap_new;
           jd.exact_ok = lr.producers == 1;
+          jd.set_words = sets ? lr.new_set.as<uint32_t>() : nullptr;
+          jd.set_bits = bits_;
           join_expand(L_, lv, cur, w, ll.cap_total, nullptr, lr.newk.as<uint64_t>(), &cnt[ri].n_new, xs,
                       &jd);
         } else {
@@ -441,17 +475,34 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
         }
       }
     }
+    // DELTA = unique(NEW) - FULL, FULL' = FULL U DELTA, DELTA's trie view
+    if (sets) {
+      for (size_t i = 0; i < X.rels.size(); i++) {
+        LoopRel& lr = X.rels[i];
+        keyset_count_dev(L_, bits_, lr.new_set.as<uint32_t>(), lr.full_set.as<uint32_t>(),
+                         lr.set_counts.as<uint32_t>());
+      }
+      // (no FULL is changed unless every relation's delta fits)
+      if (X.rels.size() > 1)
+        for (auto& lr : X.rels)
+          keyset_check_dev(L_, bits_, lr.set_counts.as<uint32_t>(), lr.cap_delta, ovf);
+    }
     for (size_t i = 0; i < X.rels.size(); i++) {
       LoopRel& lr = X.rels[i];
       LoopCounts* c = cnt + i;
-      Scratch ss{lr.sort_scr.as<char>(), lr.sort_scr.bytes(), 0};
-      // DELTA = unique(NEW) - FULL, FULL' = FULL U DELTA, DELTA's trie view
-      sort_dedup_dev(L_, lr.newk.as<uint64_t>(), lr.cap_new, &c->n_new, bits_, lr.full[p].as<uint64_t>(),
-                     lr.cap_full, &c->n_full[p], lr.delta[1 - p].as<uint64_t>(), lr.cap_delta, &c->n_delta[1 - p],
-                     ovf, ss);
-      merge_disjoint_dev(L_, lr.full[p].as<uint64_t>(), lr.cap_full, &c->n_full[p],
-                         lr.delta[1 - p].as<uint64_t>(), lr.cap_delta, &c->n_delta[1 - p],
-                         lr.full[1 - p].as<uint64_t>(), lr.cap_full, &c->n_full[1 - p], ovf);
+      if (sets) {
+        keyset_delta_dev(L_, bits_, lr.new_set.as<uint32_t>(), lr.full_set.as<uint32_t>(),
+                         lr.set_counts.as<uint32_t>(), lr.delta[1 - p].as<uint64_t>(), lr.cap_delta,
+                         &c->n_delta[1 - p], &c->n_full[p], &c->n_full[1 - p], ovf);
+      } else {
+        Scratch ss{lr.sort_scr.as<char>(), lr.sort_scr.bytes(), 0};
+        sort_dedup_dev(L_, lr.newk.as<uint64_t>(), lr.cap_new, &c->n_new, bits_, lr.full[p].as<uint64_t>(),
+                       lr.cap_full, &c->n_full[p], lr.delta[1 - p].as<uint64_t>(), lr.cap_delta, &c->n_delta[1 - p],
+                       ovf, ss);
+        merge_disjoint_dev(L_, lr.full[p].as<uint64_t>(), lr.cap_full, &c->n_full[p],
+                           lr.delta[1 - p].as<uint64_t>(), lr.cap_delta, &c->n_delta[1 - p],
+                           lr.full[1 - p].as<uint64_t>(), lr.cap_full, &c->n_full[1 - p], ovf);
+      }
       Scratch ts{lr.trie_scr.as<char>(), lr.trie_scr.bytes(), 0};
       build_trie(L_, lr.delta[1 - p].as<uint64_t>(), lr.cap_delta, lr.lo[1 - p].as<uint32_t>(),
                  lr.roots[1 - p].as<uint32_t>(), &c->n_roots[1 - p], lr.dir[1 - p].as<uint32_t>(), X.dir_n, ts,
@@ -463,10 +514,10 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
                       inst_bounds_d_.as<uint32_t>(), (uint32_t)(inst_bounds_.size() - 1), (uint32_t)(it0 + 1),
                       &X.ctl_d()->bodies, loop_marks_);
     }
-    const int ks = 2 * bits_ <= 32 ? 4 : 8;
+    const int ks = sets ? 0 : 2 * bits_ <= 32 ? 4 : 8;
     const int passes = radix_passes(L_, bits_);
-    loop_ctrl_kernel<<<1, 32, 0, L_.stream>>>(X.ctl_d(), cnt, (int)X.rels.size(), p, ks, passes, hw, hi,
-                                              set_if);
+    loop_ctrl_kernel<<<1, 32, 0, L_.stream>>>(X.ctl_d(), cnt, (int)X.rels.size(), p, ks, passes, (double)set_bytes,
+                                              hw, hi, set_if);
     SRDL_CUDA(cudaGetLastError());
     count_launches(1);
   };
@@ -590,8 +641,14 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
     r.v[kFull].clear();
     r.head = Index{};
     Index& f = r.v[kFull].idx[r.canonical];
-    f.keys = std::move(lr.full[q]);
     f.n = c.n_full[q];
+    if (sets) {
+      f.keys = DevBuf(std::max<uint64_t>(f.n, 1) * 8, L_.stream);
+      keyset_list(L_, lr.full_set.as<uint32_t>(), bits_, lr.set_counts.as<uint32_t>(), f.keys.as<uint64_t>(),
+                  d_small_.as<uint64_t>());
+    } else {
+      f.keys = std::move(lr.full[q]);
+    }
     r.v[kDelta].clear();
     r.v[kNew].clear();
     Index& d = r.v[kDelta].idx[r.canonical];

@@ -731,8 +731,13 @@ void Database::sort_into(Index& out, const uint64_t* in, uint64_t n, bool swap, 
     out.n = 0;
     return;
   }
-  DevBuf scratch(sort_scratch_bytes(n, kb), L_.stream);
+  // (room for a bitmap set where the sort would take one, unless the run's
+  // memory is limited: up to 32 MB more than the counting passes need)
+  size_t sb = sort_scratch_bytes(n, kb);
+  if (!opt_mem_limit_ && sort_by_keyset(n, kb)) sb = std::max(sb, keyset_scratch_bytes(L_, kb));
+  DevBuf scratch(sb, L_.stream);
   Scratch s{scratch.as<char>(), scratch.bytes(), 0};
+  const bool by_set = sort_by_keyset(n, kb) && keyset_scratch_bytes(L_, kb) <= sb;
   const bool hd = head && head->n;
   const bool diff = (full && full->n) || hd;
   size_t pid = prof_begin(diff ? "sort_dedup_diff" : "sort_dedup");
@@ -750,7 +755,8 @@ void Database::sort_into(Index& out, const uint64_t* in, uint64_t n, bool swap, 
     // keys once; packing reads the input; the dedup pass reads the sorted
     // keys and writes the distinct ones (plus one probe word per key into
     // FULL when the delta is fused).
-    const double ks = 2 * kb <= 32 ? 4 : 8;
+    // A bitmap set reads the keys (and FULL) once and writes the distinct ones.
+    const double ks = by_set ? 0 : 2 * kb <= 32 ? 4 : 8;
     const double passes = radix_passes(L_, kb);
     kev_[pid].bytes = passes * 2 * ks * n + 8.0 * n + ks * n + ks * n + 8.0 * out.n +
                       (diff ? 8.0 * n : 0);

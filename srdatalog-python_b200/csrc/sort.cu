@@ -563,6 +563,17 @@ int radix_passes(const Launch& L, int dom_bits) {
 
 static inline bool use32(int bits) { return 2 * bits <= 32; }
 
+// A bitmap set instead of counting passes (keyset.cu) when the key space is
+// small enough and the keys are not too few for it: clearing, counting and
+// listing 2^28 bits take about 50 us, a sort of a few ten thousand keys 75-90.
+// Measured, set / sort: 3M keys of 2^26 67 / 137 us, 20M of 2^24 174 / 470 us,
+// 200k of 2^28 53 / 91 us.
+constexpr uint64_t kKeysetSpacePerKey = 4096;
+
+bool sort_by_keyset(uint64_t n, int bits) {
+  return n > kRsSmall && 2 * bits <= kKeysetMaxBits && n >= (1ull << (2 * bits)) / kKeysetSpacePerKey;
+}
+
 size_t sort_dev_scratch_bytes(uint64_t cap, uint64_t full_cap, int bits) {
   return sort_scratch_bytes(cap, bits) + diff_dev_extra_bytes(cap, full_cap);
 }
@@ -619,6 +630,11 @@ void sort_dedup(const Launch& L, const uint64_t* in, uint64_t n, int bits, bool 
                 Scratch& s, const uint64_t* head, uint64_t n_head) {
   if (n == 0) {
     SRDL_CUDA(cudaMemsetAsync(d_nout, 0, sizeof(uint64_t), L.stream));
+    return;
+  }
+  SRDL_REQUIRE(n < (1ull << 32), kErrCapacity, "sort: more than 2^32-1 rows in one index");
+  if (sort_by_keyset(n, bits) && s.used + keyset_scratch_bytes(L, bits) <= s.cap) {
+    keyset_dedup(L, in, n, bits, swap, full, full ? n_full : 0, head, n_head, out, d_nout, s);
     return;
   }
   if (use32(bits))

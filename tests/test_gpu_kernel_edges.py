@@ -26,6 +26,20 @@ def test_sort_unique_block_edges(n, bits):
   assert np.array_equal(gpu_sort_unique(k, bits), oracle.sort_unique(k))
 
 
+# a bitmap set sorts when the key space has at most 4,096 keys per input key and
+# at most 2^28 in all
+@pytest.mark.parametrize('bits,n', [(1, 16_385), (5, 20_000), (6, 20_000), (13, 16_385), (14, 65_535), (14, 65_536),
+                                    (14, 3_000_000), (15, 3_000_000)])
+@pytest.mark.parametrize('dense', [False, True])
+def test_sort_unique_key_sets(bits, n, dense):
+  rng = np.random.default_rng(n + bits)
+  k = keys_with_bits(rng, n, bits)
+  if dense:   # a block of the key space filled, the rest nearly empty
+    k[: n - n // 16] = keys_with_bits(rng, n - n // 16, max(1, bits - 3))
+  k[n // 2] = ((1 << bits) - 1) << 32 | ((1 << bits) - 1)
+  assert np.array_equal(gpu_sort_unique(k, bits), oracle.sort_unique(k))
+
+
 @pytest.mark.parametrize('n', [5000, 300_000])
 def test_sort_unique_one_digit(n):
   '''Every key equal, then all but one (largest counters of a tile, keys of all ones).'''
@@ -33,8 +47,9 @@ def test_sort_unique_one_digit(n):
   assert np.array_equal(gpu_sort_unique(k, 32), np.array([TOP]))
   k[n // 3] = 0
   assert np.array_equal(gpu_sort_unique(k, 32), np.array([0, TOP], np.uint64))
-  k16 = np.full(n, (0xFFFF << 32) | 0xFFFF, np.uint64)   # all ones in 32-bit packed form
-  assert np.array_equal(gpu_sort_unique(k16, 16), k16[:1])
+  for bits in (14, 16):   # the largest key of a bitmap set; all ones in 32-bit packed form
+    top = np.full(n, (((1 << bits) - 1) << 32) | ((1 << bits) - 1), np.uint64)
+    assert np.array_equal(gpu_sort_unique(top, bits), top[:1])
   assert np.array_equal(gpu_sort_unique(np.sort(keys_with_bits(np.random.default_rng(n), n, 7)), 7),
                         oracle.sort_unique(keys_with_bits(np.random.default_rng(n), n, 7)))
 
