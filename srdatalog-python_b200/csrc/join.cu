@@ -52,6 +52,16 @@ __device__ __forceinline__ uint32_t rows_from(const TrieView& t, uint32_t g) {
   return (uint32_t)lower_bound_u64(t.keys, 0, t.n, (uint64_t)g << 32);
 }
 
+// in.col[k][r] with a compile-time slot index, so the Table parameter is
+// never copied to local memory for a runtime subscript.
+__device__ __forceinline__ uint32_t slot_value(const Table& t, int k, uint64_t r) {
+  uint32_t x = 0;
+#pragma unroll
+  for (int c = 0; c < kMaxSlots; c++)
+    if (c == k) x = t.col[c][r];
+  return x;
+}
+
 // List of source s for input row r: [b, b+len) over roots (no prefix), over
 // child values (prefix bound), or, for the ternary modes, over the row
 // index's children of a pair (kSrcPair) or its rows under a range of pairs
@@ -59,7 +69,7 @@ __device__ __forceinline__ uint32_t rows_from(const TrieView& t, uint32_t g) {
 __device__ __forceinline__ void src_list(const SrcSpec& s, const Table& in, uint64_t r,
                                          uint32_t& b, uint32_t& len) {
   if (s.mode == kSrcPair) {
-    const uint32_t g = pair_pos(s.pair, in.col[s.prefix_slot][r], in.col[s.prefix_slot2][r]);
+    const uint32_t g = pair_pos(s.pair, slot_value(in, s.prefix_slot, r), slot_value(in, s.prefix_slot2, r));
     uint32_t e = 0;
     b = 0;
     if (g != kNoPair) trie_range(s.t, g, b, e);
@@ -70,7 +80,7 @@ __device__ __forceinline__ void src_list(const SrcSpec& s, const Table& in, uint
       len = (uint32_t)s.t.n;
     } else {
       uint32_t kb, ke;
-      trie_range(s.pair, in.col[s.prefix_slot][r], kb, ke);
+      trie_range(s.pair, slot_value(in, s.prefix_slot, r), kb, ke);
       b = rows_from(s.t, kb);
       len = rows_from(s.t, ke) - b;
     }
@@ -79,7 +89,7 @@ __device__ __forceinline__ void src_list(const SrcSpec& s, const Table& in, uint
     len = (uint32_t)*s.t.n_roots_d;
   } else {
     uint32_t e;
-    trie_range(s.t, in.col[s.prefix_slot][r], b, e);
+    trie_range(s.t, slot_value(in, s.prefix_slot, r), b, e);
     len = e - b;
   }
 }
@@ -113,9 +123,10 @@ struct CountInit {
 constexpr int kJSmallThreads = 1024;
 constexpr uint64_t kJSmallRows = 4096;
 
-// SCAN: a single block also turns work into offs (and pwork into poffs).
-template <bool SCAN>
-__global__ void __launch_bounds__(SCAN ? kJSmallThreads : kJThreads) join_count_kernel(
+// SCAN: a single block of SCAN threads also turns work into offs (and pwork
+// into poffs).
+template <int SCAN>
+__global__ void __launch_bounds__(SCAN ? SCAN : kJThreads, SCAN ? 1 : 8) join_count_kernel(
     LevelSpec lv, Table in, uint64_t* work, uint8_t* __restrict__ drv, uint32_t* __restrict__ beg,
     uint2* __restrict__ orange, uint32_t* __restrict__ obm, uint64_t* pwork, uint64_t* offs,
     uint64_t* poffs, CountInit ci) {
@@ -173,7 +184,7 @@ __global__ void __launch_bounds__(SCAN ? kJSmallThreads : kJThreads) join_count_
         // the probed (other) list's bitmap, if its parent value has one
         const uint32_t* obd = bd ? lv.src[0].t.bdir : lv.src[1].t.bdir;
         const int ops = bd ? lv.src[0].prefix_slot : lv.src[1].prefix_slot;
-        obm[r] = (obd && ops >= 0) ? obd[in.col[ops][r]] : kNoBitmap;
+        obm[r] = (obd && ops >= 0) ? obd[slot_value(in, ops, r)] : kNoBitmap;
       }
     } else if (lv.kind == kColumnJoin) {
       uint32_t best = 0xffffffffu, bb = 0;
@@ -221,21 +232,21 @@ __global__ void __launch_bounds__(SCAN ? kJSmallThreads : kJThreads) join_count_
         work[r] = s.t.n;
       } else {
         uint32_t b, e;
-        trie_range(s.t, in.col[s.prefix_slot][r], b, e);
+        trie_range(s.t, slot_value(in, s.prefix_slot, r), b, e);
         work[r] = e - b;
       }
     }
   }
-  if constexpr (SCAN) {
-    __shared__ uint64_t sh[kJSmallThreads / 32 + 1];
+  if constexpr (SCAN > 0) {
+    __shared__ uint64_t sh[SCAN / 32 + 1];
     __syncthreads();  // this block wrote every work[r]
-    const uint64_t t = block_scan_write<kJSmallThreads>(work, (uint32_t)in.n, offs, sh);
+    const uint64_t t = block_scan_write<SCAN>(work, (uint32_t)in.n, offs, sh);
     if (threadIdx.x == 0) {
       offs[in.n] = t;
       if (ci.total) *ci.total = t;
     }
     if (pwork) {
-      const uint64_t pt = block_scan_write<kJSmallThreads>(pwork, (uint32_t)in.n, poffs, sh);
+      const uint64_t pt = block_scan_write<SCAN>(pwork, (uint32_t)in.n, poffs, sh);
       if (threadIdx.x == 0) {
         poffs[in.n] = pt;
         if (ci.ptotal) *ci.ptotal = pt;
@@ -369,16 +380,6 @@ __device__ __forceinline__ void append_key(const JoinDev& jd, unsigned m, bool o
   if (ok && (!jd.out_cap || pos < jd.out_cap)) out_keys[pos] = key;
 }
 
-// in.col[k][r] with a compile-time slot index, so the Table parameter is
-// never copied to local memory for a runtime subscript.
-__device__ __forceinline__ uint32_t slot_value(const Table& t, int k, uint64_t r) {
-  uint32_t x = 0;
-#pragma unroll
-  for (int c = 0; c < kMaxSlots; c++)
-    if (c == k) x = t.col[c][r];
-  return x;
-}
-
 __device__ __forceinline__ void slot_store(const Table& t, int k, uint64_t pos, uint32_t x) {
 #pragma unroll
   for (int c = 0; c < kMaxSlots; c++)
@@ -451,7 +452,8 @@ __global__ void __launch_bounds__(kJThreads) join_cj2_kernel(
     const uint32_t* __restrict__ beg, const uint2* __restrict__ orange,
     const uint32_t* __restrict__ obm, uint64_t total, uint64_t chunk,
     unsigned long long* __restrict__ queue, Table out, uint64_t* __restrict__ out_keys,
-    unsigned long long* __restrict__ d_out_n, uint64_t* __restrict__ chunk_counts, JoinDev jd) {
+    unsigned long long* __restrict__ d_out_n, uint64_t* __restrict__ chunk_counts, uint2* __restrict__ stage,
+    JoinDev jd) {
   const int lane = threadIdx.x & 31;
   // (count-only rules never run in the device loop: the count instance
   // keeps the registers of the hot triangle level free of it)
@@ -596,6 +598,8 @@ __global__ void __launch_bounds__(kJThreads) join_cj2_kernel(
           atomicAdd(&lv.grp_counts[g], (unsigned long long)__popc(peers));
       }
       if (MODE == kModeCount || MODE == kModeTableCount) {
+        if (MODE == kModeTableCount && stage && ok)
+          stage[c0 + running + __popc(m & lanemask_lt())] = make_uint2((uint32_t)r, v);
         running += __popc(m);
       } else if (MODE == kModeKeys) {
         uint64_t key = 0;
@@ -625,6 +629,37 @@ __global__ void __launch_bounds__(kJThreads) join_cj2_kernel(
     else if (MODE == kModeTableCount && lane == 0) chunk_counts[k] = running;
   }
   if (MODE == kModeCount && lane == 0 && counted) atomicAdd(d_out_n, counted);
+}
+
+// Tables of few candidates: the count pass also left each chunk's survivors
+// (input row, value) at the chunk's own place, and this launch moves them to
+// their final place, one warp per chunk, every block adding up the counts of
+// the chunks before its own.  Probing the candidates once and scanning the
+// counts here takes two launches of a few microseconds where the scanned form
+// takes three (8 + 4 + 9 us for a table of some thousand candidates).
+constexpr uint64_t kCj2StageTotal = 1u << 17;  // candidates
+__global__ void __launch_bounds__(kJThreads) join_stage_kernel(LevelSpec lv, Table in, const uint2* __restrict__ stage,
+                                                               const uint64_t* __restrict__ chunk_counts,
+                                                               uint64_t nchunks, uint64_t chunk, Table out,
+                                                               unsigned long long* __restrict__ d_out_n) {
+  __shared__ uint64_t sh[kJThreads / 32 + 1];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const uint64_t k0 = (uint64_t)blockIdx.x * (kJThreads / 32);
+  uint64_t pos = block_prefix(chunk_counts, (uint32_t)k0, sh);
+  uint64_t cnt = 0;
+  for (int w = 0; w < kJThreads / 32; w++) {
+    const uint64_t c = k0 + w < nchunks ? chunk_counts[k0 + w] : 0;
+    if (w < wid) pos += c;
+    if (w == wid) cnt = c;
+  }
+  if (blockIdx.x == gridDim.x - 1 && wid == kJThreads / 32 - 1 && lane == 0) *d_out_n = pos + cnt;
+  for (uint64_t i = lane; i < cnt; i += 32) {
+    const uint2 e = stage[(k0 + wid) * chunk + i];
+#pragma unroll
+    for (int c = 0; c < kMaxSlots; c++)
+      if (c < lv.n_in_slots) out.col[c][pos + i] = in.col[c][e.x];
+    slot_store(out, lv.cj_slot, pos + i, e.y);
+  }
 }
 
 template <int MODE, bool SEG>
@@ -867,7 +902,9 @@ size_t join_expand_scratch_bytes(const Launch& L, uint64_t total) {
   const uint64_t warps = (uint64_t)jgrid(total, L) * (kJThreads / 32);
   const uint64_t chunks = std::min<uint64_t>(kCj2MaxTableChunks, (total + 63) / 64);
   const uint64_t n = std::max<uint64_t>(warps, chunks);
-  return 2 * ((n + 1) * 8 + 255) + scan_scratch_bytes(n) + 4096;
+  // (+ the staged survivors of a small table)
+  const uint64_t staged = total <= kCj2StageTotal ? total * 8 + 256 : 0;
+  return 2 * ((n + 1) * 8 + 255) + scan_scratch_bytes(n) + 4096 + staged;
 }
 
 // Resident blocks per SM of the two-source column-join kernel for a level
@@ -1146,14 +1183,18 @@ JoinWork join_count(const Launch& L, const LevelSpec& lv, const Table& in, Scrat
   }
   CountInit ci{w.queue, zero, total, ptotal};
   if (in.n && in.n <= kJSmallRows) {
-    join_count_kernel<true><<<1, kJSmallThreads, 0, L.stream>>>(lv, in, work, w.drv, w.beg, w.orange, w.obm, pwork,
-                                                                w.offs, w.poffs, ci);
+    if (in.n <= 4 * kJThreads)
+      join_count_kernel<kJThreads><<<1, kJThreads, 0, L.stream>>>(lv, in, work, w.drv, w.beg, w.orange, w.obm, pwork,
+                                                                  w.offs, w.poffs, ci);
+    else
+      join_count_kernel<kJSmallThreads><<<1, kJSmallThreads, 0, L.stream>>>(lv, in, work, w.drv, w.beg, w.orange,
+                                                                            w.obm, pwork, w.offs, w.poffs, ci);
     SRDL_CUDA(cudaGetLastError());
     count_launches(1);
     return w;
   }
   if (in.n) {
-    join_count_kernel<false><<<jgrid(in.n, L), kJThreads, 0, L.stream>>>(lv, in, work, w.drv, w.beg, w.orange, w.obm,
+    join_count_kernel<0><<<jgrid(in.n, L), kJThreads, 0, L.stream>>>(lv, in, work, w.drv, w.beg, w.orange, w.obm,
                                                                          pwork, nullptr, nullptr, ci);
     SRDL_CUDA(cudaGetLastError());
     count_launches(1);
@@ -1242,26 +1283,33 @@ void join_expand(const Launch& L, const LevelSpec& lv, const Table& in, const Jo
                                                (nchunks + kJThreads / 32 - 1) / (kJThreads / 32));
     const int gq = (int)std::max<uint64_t>(blocks, 1);
     unsigned long long* q = w.queue;  // zeroed by the count launch
-#define SRDL_CJ2(MODE, Q, CC)                                                                     \
+#define SRDL_CJ2(MODE, Q, CC, ST)                                                                 \
   (lv.seg ? join_cj2_kernel<MODE, true><<<gq, kJThreads, 0, L.stream>>>(                           \
                 lv, in, w.offs, w.drv, w.beg, w.orange, w.obm, total, chunk, Q, out, out_keys, cnt, \
-                CC, jd)                                                                           \
+                CC, ST, jd)                                                                       \
           : join_cj2_kernel<MODE, false><<<gq, kJThreads, 0, L.stream>>>(                          \
                 lv, in, w.offs, w.drv, w.beg, w.orange, w.obm, total, chunk, Q, out, out_keys, cnt, \
-                CC, jd))
+                CC, ST, jd))
     if (lv.emit == kEmitCount) {
-      SRDL_CJ2(kModeCount, q, nullptr);
+      SRDL_CJ2(kModeCount, q, nullptr, nullptr);
       count_launches(1);
     } else if (lv.emit == kEmitKeys) {
-      SRDL_CJ2(kModeKeys, q, nullptr);
+      SRDL_CJ2(kModeKeys, q, nullptr, nullptr);
       count_launches(1);
     } else {
       uint64_t* cc = s.take<uint64_t>(nchunks + 1);
-      uint64_t* co = s.take<uint64_t>(nchunks + 1);
-      SRDL_CJ2(kModeTableCount, q, cc);
-      SRDL_CUDA(cudaGetLastError());
-      exclusive_scan_u64(L, cc, nchunks, co, s, d_out_n);
-      SRDL_CJ2(kModeTableWrite, q + 1, co);
+      if (total <= kCj2StageTotal) {
+        uint2* st = s.take<uint2>(total);
+        SRDL_CJ2(kModeTableCount, q, cc, st);
+        join_stage_kernel<<<(unsigned)((nchunks + kJThreads / 32 - 1) / (kJThreads / 32)), kJThreads, 0, L.stream>>>(
+            lv, in, st, cc, nchunks, chunk, out, cnt);
+      } else {
+        uint64_t* co = s.take<uint64_t>(nchunks + 1);
+        SRDL_CJ2(kModeTableCount, q, cc, nullptr);
+        SRDL_CUDA(cudaGetLastError());
+        exclusive_scan_u64(L, cc, nchunks, co, s, d_out_n);
+        SRDL_CJ2(kModeTableWrite, q + 1, co, nullptr);
+      }
       count_launches(2);
     }
 #undef SRDL_CJ2
