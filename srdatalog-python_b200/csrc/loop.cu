@@ -29,7 +29,9 @@
 // lacks are listed as DELTA and added to FULL, and FULL is listed as a sorted
 // array once, after the last iteration -- no rule of a qualifying step reads it
 // before.  That takes the place of the sort, the set difference and the merge
-// of every iteration.  On overflow the failed iteration's inputs are
+// of every iteration.  DELTA is written after the joins have read the one
+// before, so one buffer set is enough and the graph is WHILE (go) { iteration;
+// control }, half as long to capture and instantiate.  On overflow the failed iteration's inputs are
 // intact (they are the other buffer set): the host resumes from them on the
 // host path, and the next entry sizes the buffers from the larger counts
 // that path measures.  Results are those of the host path: the same
@@ -65,7 +67,8 @@ struct LoopCtl {
 };
 
 // ks: packed key bytes of the sort, passes: its counting passes.
-// (ks 0: bitmap sets of set_bytes each)
+// (ks 0: bitmap sets of set_bytes each, one buffer set: the iteration's counts
+// at index 1 become those at index 0)
 __global__ void loop_ctrl_kernel(LoopCtl* ctl, LoopCounts* cnt, int nrel, int p, int ks, int passes,
                                  double set_bytes, cudaGraphConditionalHandle hw, cudaGraphConditionalHandle hi,
                                  int set_if) {
@@ -74,7 +77,7 @@ __global__ void loop_ctrl_kernel(LoopCtl* ctl, LoopCounts* cnt, int nrel, int p,
   unsigned go = 0;
   if (!ctl->overflow) {
     ctl->done++;
-    ctl->parity = 1 - p;
+    ctl->parity = ks ? 1 - p : 0;
     uint64_t delta = 0;
     for (int r = 0; r < nrel; r++) {
       const double nn = (double)cnt[r].n_new, nd = (double)cnt[r].n_delta[1 - p];
@@ -88,6 +91,11 @@ __global__ void loop_ctrl_kernel(LoopCtl* ctl, LoopCounts* cnt, int nrel, int p,
                           8.0 * nn + 16.0 * (nf + nd) + 16.0 * nd;
       else
         ctl->alg_bytes += 8.0 * nn + 2.0 * set_bytes + 8.0 * nd + 16.0 * nd;
+      if (!ks) {
+        cnt[r].n_full[0] = cnt[r].n_full[1];
+        cnt[r].n_delta[0] = cnt[r].n_delta[1];
+        cnt[r].n_roots[0] = cnt[r].n_roots[1];
+      }
     }
     go = delta > 0 && ctl->done < ctl->remaining;
   }
@@ -271,7 +279,7 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
       {
         // the buffers below; leave the step to the host path rather than
         // take most of the free memory (the host path needs far less)
-        const uint64_t need = lr.cap_delta * (16 + 8 + 8) +
+        const uint64_t need = lr.cap_delta * (sets ? 16 : 16 + 8 + 8) +
                               (sets ? 2 * set_bytes
                                     : lr.cap_new * 8 + lr.cap_full * 16 +
                                           sort_dev_scratch_bytes(lr.cap_new, lr.cap_full, bits_));
@@ -291,7 +299,7 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
         lr.sort_scr = DevBuf(sort_dev_scratch_bytes(lr.cap_new, lr.cap_full, bits_), L_.stream);
       }
       lr.trie_scr = DevBuf(trie_scratch_bytes(lr.cap_delta) + 1024, L_.stream);
-      for (int q = 0; q < 2; q++) {
+      for (int q = 0; q < (sets ? 1 : 2); q++) {
         if (!sets) lr.full[q] = DevBuf(lr.cap_full * 8, L_.stream);
         lr.delta[q] = DevBuf(lr.cap_delta * 8, L_.stream);
         lr.lo[q] = DevBuf(lr.cap_delta * 4, L_.stream);
@@ -419,8 +427,10 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
     }
   }
 
-  // ---- one iteration reading buffer set p, writing 1 - p, then the control kernel
+  // ---- one iteration reading buffer set p, writing 1 - p (bitmap sets: p = 0,
+  // written in place), then the control kernel
   auto body = [&](int p, cudaGraphConditionalHandle hw, cudaGraphConditionalHandle hi, int set_if) {
+    const int o = sets ? 0 : 1 - p;
     LoopCounts* cnt = X.cnt_d();
     unsigned int* ovf = &X.ctl_d()->overflow;
     std::vector<char> zeroed(X.rels.size(), 0);  // n_new of the relations a rule has begun to fill
@@ -492,25 +502,25 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
       LoopCounts* c = cnt + i;
       if (sets) {
         keyset_delta_dev(L_, bits_, lr.new_set.as<uint32_t>(), lr.full_set.as<uint32_t>(),
-                         lr.set_counts.as<uint32_t>(), lr.delta[1 - p].as<uint64_t>(), lr.cap_delta,
+                         lr.set_counts.as<uint32_t>(), lr.delta[o].as<uint64_t>(), lr.cap_delta,
                          &c->n_delta[1 - p], &c->n_full[p], &c->n_full[1 - p], ovf);
       } else {
         Scratch ss{lr.sort_scr.as<char>(), lr.sort_scr.bytes(), 0};
         sort_dedup_dev(L_, lr.newk.as<uint64_t>(), lr.cap_new, &c->n_new, bits_, lr.full[p].as<uint64_t>(),
-                       lr.cap_full, &c->n_full[p], lr.delta[1 - p].as<uint64_t>(), lr.cap_delta, &c->n_delta[1 - p],
+                       lr.cap_full, &c->n_full[p], lr.delta[o].as<uint64_t>(), lr.cap_delta, &c->n_delta[1 - p],
                        ovf, ss);
         merge_disjoint_dev(L_, lr.full[p].as<uint64_t>(), lr.cap_full, &c->n_full[p],
-                           lr.delta[1 - p].as<uint64_t>(), lr.cap_delta, &c->n_delta[1 - p],
+                           lr.delta[o].as<uint64_t>(), lr.cap_delta, &c->n_delta[1 - p],
                            lr.full[1 - p].as<uint64_t>(), lr.cap_full, &c->n_full[1 - p], ovf);
       }
       Scratch ts{lr.trie_scr.as<char>(), lr.trie_scr.bytes(), 0};
-      build_trie(L_, lr.delta[1 - p].as<uint64_t>(), lr.cap_delta, lr.lo[1 - p].as<uint32_t>(),
-                 lr.roots[1 - p].as<uint32_t>(), &c->n_roots[1 - p], lr.dir[1 - p].as<uint32_t>(), X.dir_n, ts,
+      build_trie(L_, lr.delta[o].as<uint64_t>(), lr.cap_delta, lr.lo[o].as<uint32_t>(),
+                 lr.roots[o].as<uint32_t>(), &c->n_roots[1 - p], lr.dir[o].as<uint32_t>(), X.dir_n, ts,
                  &c->n_delta[1 - p]);
       // batched runs: the instances with a delta row in this iteration
       // (its number is it0 + 1 + the bodies started before it)
       if (loop_marks_)
-        instance_mark(L_, lr.delta[1 - p].as<uint64_t>(), lr.cap_delta, &c->n_delta[1 - p],
+        instance_mark(L_, lr.delta[o].as<uint64_t>(), lr.cap_delta, &c->n_delta[1 - p],
                       inst_bounds_d_.as<uint32_t>(), (uint32_t)(inst_bounds_.size() - 1), (uint32_t)(it0 + 1),
                       &X.ctl_d()->bodies, loop_marks_);
     }
@@ -556,9 +566,9 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
   uint64_t per_body = 0;
   try {
     SRDL_CUDA(cudaGraphCreate(&g, 0));
-    cudaGraphConditionalHandle hw, hi;
+    cudaGraphConditionalHandle hw, hi{};
     SRDL_CUDA(cudaGraphConditionalHandleCreate(&hw, g, 1, cudaGraphCondAssignDefault));
-    SRDL_CUDA(cudaGraphConditionalHandleCreate(&hi, g, 0, cudaGraphCondAssignDefault));
+    if (!sets) SRDL_CUDA(cudaGraphConditionalHandleCreate(&hi, g, 0, cudaGraphCondAssignDefault));
     cudaGraphNodeParams wp = {};
     wp.type = cudaGraphNodeTypeConditional;
     wp.conditional.handle = hw;
@@ -571,35 +581,39 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
     SRDL_CUDA(cudaStreamBeginCaptureToGraph(L_.stream, wbody, nullptr, nullptr, 0,
                                             cudaStreamCaptureModeThreadLocal));
     try {
-      body(0, hw, hi, 1);
+      body(0, hw, hi, sets ? 0 : 1);
     } catch (...) {
       cudaStreamEndCapture(L_.stream, &tmp);
       throw;
     }
     per_body = launches_total() - l0;
-    cudaStreamCaptureStatus cs;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t ndeps = 0;
-    SRDL_CUDA(cudaStreamGetCaptureInfo(L_.stream, &cs, nullptr, nullptr, &deps, &ndeps));
-    std::vector<cudaGraphNode_t> tail(deps, deps + ndeps);
-    SRDL_CUDA(cudaStreamEndCapture(L_.stream, &tmp));
-    cudaGraphNodeParams ip = {};
-    ip.type = cudaGraphNodeTypeConditional;
-    ip.conditional.handle = hi;
-    ip.conditional.type = cudaGraphCondTypeIf;
-    ip.conditional.size = 1;
-    cudaGraphNode_t inode;
-    SRDL_CUDA(cudaGraphAddNode(&inode, wbody, tail.data(), tail.size(), &ip));
-    cudaGraph_t ibody = ip.conditional.phGraph_out[0];
-    SRDL_CUDA(cudaStreamBeginCaptureToGraph(L_.stream, ibody, nullptr, nullptr, 0,
-                                            cudaStreamCaptureModeThreadLocal));
-    try {
-      body(1, hw, hi, 0);
-    } catch (...) {
-      cudaStreamEndCapture(L_.stream, &tmp);
-      throw;
+    if (sets) {
+      SRDL_CUDA(cudaStreamEndCapture(L_.stream, &tmp));
+    } else {
+      cudaStreamCaptureStatus cs;
+      const cudaGraphNode_t* deps = nullptr;
+      size_t ndeps = 0;
+      SRDL_CUDA(cudaStreamGetCaptureInfo(L_.stream, &cs, nullptr, nullptr, &deps, &ndeps));
+      std::vector<cudaGraphNode_t> tail(deps, deps + ndeps);
+      SRDL_CUDA(cudaStreamEndCapture(L_.stream, &tmp));
+      cudaGraphNodeParams ip = {};
+      ip.type = cudaGraphNodeTypeConditional;
+      ip.conditional.handle = hi;
+      ip.conditional.type = cudaGraphCondTypeIf;
+      ip.conditional.size = 1;
+      cudaGraphNode_t inode;
+      SRDL_CUDA(cudaGraphAddNode(&inode, wbody, tail.data(), tail.size(), &ip));
+      cudaGraph_t ibody = ip.conditional.phGraph_out[0];
+      SRDL_CUDA(cudaStreamBeginCaptureToGraph(L_.stream, ibody, nullptr, nullptr, 0,
+                                              cudaStreamCaptureModeThreadLocal));
+      try {
+        body(1, hw, hi, 0);
+      } catch (...) {
+        cudaStreamEndCapture(L_.stream, &tmp);
+        throw;
+      }
+      SRDL_CUDA(cudaStreamEndCapture(L_.stream, &tmp));
     }
-    SRDL_CUDA(cudaStreamEndCapture(L_.stream, &tmp));
     SRDL_CUDA(cudaGraphInstantiate(&ge, g, 0));
   } catch (const Error& e) {
     // a capture the runtime refuses leaves the step to the host path
@@ -662,6 +676,14 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
     SRDL_CUDA(cudaMemcpyAsync(d.nroots_d.as<void>(), &X.cnt_d()[i].n_roots[q], 8, cudaMemcpyDeviceToDevice,
                               L_.stream));
     d.trie = true;
+    if (sets && ctl.overflow) {
+      // (the failed iteration's empty delta has replaced the trie view)
+      d.lo.reset();
+      d.roots.reset();
+      d.dir.reset();
+      d.nroots_d.reset();
+      d.trie = false;
+    }
     r.delta_epoch += ctl.done;
     r.base_epoch = r.delta_epoch - 1;
     r.full_epoch = r.delta_epoch;
