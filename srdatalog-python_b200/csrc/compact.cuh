@@ -168,7 +168,10 @@ void compact(const Launch& L, Sel sel, uint64_t n, uint64_t* d_total, Scratch& s
 // sorted unique arrays full[0..n_full) and head[0..n_head) (a Device2Level
 // relation's two segments; head may be empty).  Keys are stored compressed
 // as (hi << bits) | lo and are expanded to (hi << 32) | lo on output.
-template <typename K>
+// PLAIN: the keys are whole (bits = 32) and distinct, known at compile time --
+// the standalone set difference, whose mark pass is bound by instructions: 322
+// us for 50M - 30M keys, 363 when it expanded and compared them as the sort's.
+template <typename K, bool PLAIN = false>
 struct DedupDiffSel {
   const K* a;
   int bits;
@@ -183,13 +186,14 @@ struct DedupDiffSel {
   unsigned int* d_overflow = nullptr;
 
   __device__ __forceinline__ uint64_t expand(K c) const {
-    if (sizeof(K) == 8 && bits == 32) return (uint64_t)c;
+    if (PLAIN || (sizeof(K) == 8 && bits == 32)) return (uint64_t)c;
     const uint64_t m = (1ull << bits) - 1;
     return (((uint64_t)c >> bits) << 32) | ((uint64_t)c & m);
   }
   __device__ void block_setup(uint64_t, uint64_t) {}
   // (without FULL and HEAD: compact_diff takes the paths below otherwise)
-  __device__ bool select(uint64_t i) const { return !(dedup && i > 0 && a[i - 1] == a[i]); }
+  __device__ __forceinline__ bool repeats(K before, K key) const { return !PLAIN && dedup && before == key; }
+  __device__ bool select(uint64_t i) const { return !(i > 0 && repeats(a[i - 1], a[i])); }
   using value_type = uint64_t;
   __device__ uint64_t value(uint64_t i) const { return expand(a[i]); }
   __device__ void store(uint64_t pos, uint64_t v) const {
@@ -204,8 +208,8 @@ struct DedupDiffSel {
 // search in FULL per key and nothing else.
 enum DiffPath : int { kPathAny = 0, kPathMerge = 1, kPathProbe = 2 };
 
-template <typename K>
-__device__ __forceinline__ bool diff_path_runs(int path, const DedupDiffSel<K>& sel, uint64_t n) {
+template <typename K, bool PLAIN>
+__device__ __forceinline__ bool diff_path_runs(int path, const DedupDiffSel<K, PLAIN>& sel, uint64_t n) {
   if (path == kPathAny) return true;
   const bool merge = sel.n_full <= kDmMaxFullRatio * n;
   return (path == kPathMerge) == merge;
@@ -238,8 +242,8 @@ __device__ __forceinline__ void dd_lower_bounds(const uint64_t* __restrict__ a, 
 // neighbours, so the last steps of a round's searches share lines.  30k keys
 // against 8M: 50 us for the whole set difference, 103 us with eight searches
 // one after another per thread.
-template <typename K>
-__global__ void __launch_bounds__(kCpThreads) dd_probe_kernel(DedupDiffSel<K> sel, uint64_t n, uint64_t chunk,
+template <typename K, bool PLAIN>
+__global__ void __launch_bounds__(kCpThreads) dd_probe_kernel(DedupDiffSel<K, PLAIN> sel, uint64_t n, uint64_t chunk,
                                                               uint32_t* __restrict__ flags,
                                                               uint32_t* __restrict__ blk_counts,
                                                               const uint64_t* d_n, int path) {
@@ -260,7 +264,7 @@ __global__ void __launch_bounds__(kCpThreads) dd_probe_kernel(DedupDiffSel<K> se
     for (int q = 0; q < kDdKeys; q++) {
       const uint64_t i = w0 + q * 32 + lane;
       const K c = i < end ? sel.a[i] : K(0);
-      keep[q] = i < end && !(sel.dedup && i > 0 && sel.a[i - 1] == c);
+      keep[q] = i < end && !(i > 0 && !PLAIN && sel.repeats(sel.a[i - 1], c));
       k[q] = sel.expand(c);
     }
     if (sel.n_full) {
@@ -300,8 +304,8 @@ __global__ void __launch_bounds__(kCpThreads) dd_probe_kernel(DedupDiffSel<K> se
 // start on a word boundary).
 
 // Number of a-keys among the first `diag` merged elements.
-template <typename K>
-__device__ __forceinline__ uint64_t dm_path(const DedupDiffSel<K>& sel, uint64_t na,
+template <typename K, bool PLAIN>
+__device__ __forceinline__ uint64_t dm_path(const DedupDiffSel<K, PLAIN>& sel, uint64_t na,
                                             uint64_t diag) {
   uint64_t lo = diag > sel.n_full ? diag - sel.n_full : 0;
   uint64_t hi = diag < na ? diag : na;
@@ -315,8 +319,8 @@ __device__ __forceinline__ uint64_t dm_path(const DedupDiffSel<K>& sel, uint64_t
 
 // split[t] = a-keys among the first t*kCpTile merged elements; hpos[t] = the
 // HEAD position of a[split[t]] (n_head past the last key).
-template <typename K>
-__global__ void dm_split_kernel(DedupDiffSel<K> sel, uint64_t na, uint64_t tiles,
+template <typename K, bool PLAIN>
+__global__ void dm_split_kernel(DedupDiffSel<K, PLAIN> sel, uint64_t na, uint64_t tiles,
                                 uint64_t* __restrict__ split, uint64_t* __restrict__ hpos,
                                 const uint64_t* d_n, int path) {
   const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
@@ -342,8 +346,8 @@ __device__ __forceinline__ void cp_async_small(void* smem, const void* gmem) {
 
 // One merged tile's slices: la a-keys (K) at the start of the buffer, lf FULL
 // keys after them at an 8-byte boundary; returns nothing, commits one group.
-template <typename K>
-__device__ __forceinline__ void dm_fetch(const DedupDiffSel<K>& sel, unsigned char* buf,
+template <typename K, bool PLAIN>
+__device__ __forceinline__ void dm_fetch(const DedupDiffSel<K, PLAIN>& sel, unsigned char* buf,
                                          uint64_t i0, uint32_t la, uint64_t j0, uint32_t lf) {
   K* da = reinterpret_cast<K*>(buf);
   uint64_t* df = reinterpret_cast<uint64_t*>(buf + ((la * sizeof(K) + 7) & ~size_t(7)));
@@ -352,8 +356,8 @@ __device__ __forceinline__ void dm_fetch(const DedupDiffSel<K>& sel, unsigned ch
   asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
 
-template <typename K>
-__global__ void __launch_bounds__(kCpThreads) dm_mark_kernel(DedupDiffSel<K> sel, uint64_t na,
+template <typename K, bool PLAIN>
+__global__ void __launch_bounds__(kCpThreads) dm_mark_kernel(DedupDiffSel<K, PLAIN> sel, uint64_t na,
                                                              uint64_t tiles,
                                                              const uint64_t* __restrict__ split,
                                                              const uint64_t* __restrict__ hpos,
@@ -432,7 +436,7 @@ __global__ void __launch_bounds__(kCpThreads) dm_mark_kernel(DedupDiffSel<K> sel
           has_f = true;
           continue;
         }
-        bool keep = !(has_f && last_f == x) && !(sel.dedup && has_p && prev == x);
+        bool keep = !(has_f && last_f == x) && (PLAIN || !(sel.dedup && has_p && prev == x));
         if (keep && h1 > h0) {
           const uint64_t g = lower_bound_u64(sel.head, h0, h1, x);
           keep = !(g < h1 && sel.head[g] == x);
@@ -460,11 +464,11 @@ __global__ void __launch_bounds__(kCpThreads) dm_mark_kernel(DedupDiffSel<K> sel
 }
 
 // Per-block selected counts of a flag-word array (blocks own `chunk` keys).
-template <typename K>
+template <typename K, bool PLAIN>
 static __global__ void __launch_bounds__(kCpThreads) cp_count_kernel(const uint32_t* __restrict__ flags,
                                                               uint64_t n, uint64_t chunk,
                                                               uint32_t* blk_counts,
-                                                              DedupDiffSel<K> sel,
+                                                              DedupDiffSel<K, PLAIN> sel,
                                                               const uint64_t* d_n, int path) {
   __shared__ uint32_t sh[kCpThreads / 32 + 1];
   sel.n_full = dev_size(sel.n_full, sel.d_n_full);
@@ -483,8 +487,8 @@ static __global__ void __launch_bounds__(kCpThreads) cp_count_kernel(const uint3
 
 // compact() for DedupDiffSel with a FULL array: merge path when FULL is not
 // much larger than the keys, one search per key otherwise.
-template <typename K>
-void compact_diff(const Launch& L, DedupDiffSel<K> sel, uint64_t n, uint64_t* d_total, Scratch& s) {
+template <typename K, bool PLAIN>
+void compact_diff(const Launch& L, DedupDiffSel<K, PLAIN> sel, uint64_t n, uint64_t* d_total, Scratch& s) {
   if (!sel.head || sel.n_head == 0) {
     sel.head = nullptr;
     sel.n_head = 0;
@@ -504,17 +508,17 @@ void compact_diff(const Launch& L, DedupDiffSel<K> sel, uint64_t n, uint64_t* d_
     uint64_t* split = s.take<uint64_t>(mtiles + 1);
     uint64_t* mhpos = sel.head ? s.take<uint64_t>(mtiles + 1) : nullptr;
     SRDL_CUDA(cudaMemsetAsync(flags, 0, cp_words(n) * 4, L.stream));
-    dm_split_kernel<K><<<(unsigned)((mtiles + 1 + 255) / 256), 256, 0, L.stream>>>(sel, n, mtiles, split, mhpos,
+    dm_split_kernel<K, PLAIN><<<(unsigned)((mtiles + 1 + 255) / 256), 256, 0, L.stream>>>(sel, n, mtiles, split, mhpos,
                                                                                   nullptr, kPathAny);
     const unsigned mgrid = (unsigned)std::min<uint64_t>(mtiles, (uint64_t)L.num_sms * 4);
-    dm_mark_kernel<K><<<mgrid, kCpThreads, 0, L.stream>>>(sel, n, mtiles, split, mhpos, flags, nullptr, kPathAny);
-    cp_count_kernel<K><<<nb, kCpThreads, 0, L.stream>>>(flags, n, chunk, counts, sel, nullptr, kPathAny);
+    dm_mark_kernel<K, PLAIN><<<mgrid, kCpThreads, 0, L.stream>>>(sel, n, mtiles, split, mhpos, flags, nullptr, kPathAny);
+    cp_count_kernel<K, PLAIN><<<nb, kCpThreads, 0, L.stream>>>(flags, n, chunk, counts, sel, nullptr, kPathAny);
     count_launches(3);
   } else {
-    dd_probe_kernel<K><<<nb, kCpThreads, 0, L.stream>>>(sel, n, chunk, flags, counts, nullptr, kPathAny);
+    dd_probe_kernel<K, PLAIN><<<nb, kCpThreads, 0, L.stream>>>(sel, n, chunk, flags, counts, nullptr, kPathAny);
     count_launches(1);
   }
-  cp_write_kernel<DedupDiffSel<K>><<<nb, kCpThreads, 0, L.stream>>>(sel, n, chunk, flags, counts, d_total, nullptr);
+  cp_write_kernel<DedupDiffSel<K, PLAIN>><<<nb, kCpThreads, 0, L.stream>>>(sel, n, chunk, flags, counts, d_total, nullptr);
   SRDL_CUDA(cudaGetLastError());
   count_launches(1);
 }
@@ -529,8 +533,8 @@ inline size_t diff_dev_extra_bytes(uint64_t cap, uint64_t full_cap) {
   return ((cap + full_cap) / kCpTile + 2) * 8 + 512;
 }
 
-template <typename K>
-void compact_diff_dev(const Launch& L, DedupDiffSel<K> sel, uint64_t cap, const uint64_t* d_n,
+template <typename K, bool PLAIN>
+void compact_diff_dev(const Launch& L, DedupDiffSel<K, PLAIN> sel, uint64_t cap, const uint64_t* d_n,
                       uint64_t* d_total, Scratch& s) {
   sel.head = nullptr;
   sel.n_head = 0;
@@ -549,15 +553,15 @@ void compact_diff_dev(const Launch& L, DedupDiffSel<K> sel, uint64_t cap, const 
   uint64_t* split = s.take<uint64_t>(mtiles + 1);
   // merge path: the mark pass ORs its bits into zeroed flag words
   SRDL_CUDA(cudaMemsetAsync(flags, 0, cp_words(cap) * 4, L.stream));
-  dm_split_kernel<K><<<(unsigned)((mtiles + 1 + 255) / 256), 256, 0, L.stream>>>(sel, cap, mtiles, split, nullptr,
+  dm_split_kernel<K, PLAIN><<<(unsigned)((mtiles + 1 + 255) / 256), 256, 0, L.stream>>>(sel, cap, mtiles, split, nullptr,
                                                                                 d_n, kPathMerge);
   const unsigned mgrid = (unsigned)std::min<uint64_t>(mtiles, (uint64_t)L.num_sms * 4);
-  dm_mark_kernel<K><<<mgrid, kCpThreads, 0, L.stream>>>(sel, cap, mtiles, split, nullptr, flags, d_n, kPathMerge);
-  cp_count_kernel<K><<<nb, kCpThreads, 0, L.stream>>>(flags, cap, 0, counts, sel, d_n, kPathMerge);
+  dm_mark_kernel<K, PLAIN><<<mgrid, kCpThreads, 0, L.stream>>>(sel, cap, mtiles, split, nullptr, flags, d_n, kPathMerge);
+  cp_count_kernel<K, PLAIN><<<nb, kCpThreads, 0, L.stream>>>(flags, cap, 0, counts, sel, d_n, kPathMerge);
   // probe path
-  dd_probe_kernel<K><<<nb, kCpThreads, 0, L.stream>>>(sel, cap, 0, flags, counts, d_n, kPathProbe);
+  dd_probe_kernel<K, PLAIN><<<nb, kCpThreads, 0, L.stream>>>(sel, cap, 0, flags, counts, d_n, kPathProbe);
   // either way: the ordered write of the kept keys
-  cp_write_kernel<DedupDiffSel<K>><<<nb, kCpThreads, 0, L.stream>>>(sel, cap, 0, flags, counts, d_total, d_n);
+  cp_write_kernel<DedupDiffSel<K, PLAIN>><<<nb, kCpThreads, 0, L.stream>>>(sel, cap, 0, flags, counts, d_total, d_n);
   SRDL_CUDA(cudaGetLastError());
   count_launches(5);
 }

@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(kKsThreads) ks_add_kernel(const uint64_t* __re
   const uint64_t step = (uint64_t)gridDim.x * kKsThreads;
   auto place = [&](uint64_t k) -> uint32_t {
     const uint32_t hi = swap ? (uint32_t)k : (uint32_t)(k >> 32), lo = swap ? (uint32_t)(k >> 32) : (uint32_t)k;
-    return (hi << bits) | lo;
+    return ((hi << bits) | lo) & ((1u << (2 * bits)) - 1);  // (values past `bits` bits must not leave the set)
   };
   auto add = [&](uint32_t p) { atomicOr(words + (p >> 5), 1u << (p & 31)); };
   uint64_t i = blockIdx.x * (uint64_t)kKsThreads + threadIdx.x;
@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(kKsThreads) ks_sorted_kernel(const uint64_t* _
     uint32_t w = 0xffffffffu, b = 0;
     if (i < n) {
       const uint64_t k = __ldg(keys + i);
-      const uint32_t p = ((uint32_t)(k >> 32) << bits) | (uint32_t)k;
+      const uint32_t p = (((uint32_t)(k >> 32) << bits) | (uint32_t)k) & ((1u << (2 * bits)) - 1);
       w = p >> 5;
       b = 1u << (p & 31);
     }

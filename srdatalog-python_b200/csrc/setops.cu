@@ -181,7 +181,7 @@ size_t diff_scratch_bytes(uint64_t n) { return cp_scratch_bytes(n); }
 
 void set_difference(const Launch& L, const uint64_t* a, uint64_t na, const uint64_t* b,
                     uint64_t nb, uint64_t* out, uint64_t* d_nout, Scratch& s) {
-  DedupDiffSel<uint64_t> sel{a, 32, false, b, nb, out};
+  DedupDiffSel<uint64_t, true> sel{a, 32, false, b, nb, out};
   compact_diff(L, sel, na, d_nout, s);
 }
 

@@ -566,12 +566,15 @@ static inline bool use32(int bits) { return 2 * bits <= 32; }
 // A bitmap set instead of counting passes (keyset.cu) when the key space is
 // small enough and the keys are not too few for it: clearing, counting and
 // listing 2^28 bits take about 50 us, a sort of a few ten thousand keys 75-90.
-// Measured, set / sort: 3M keys of 2^26 67 / 137 us, 20M of 2^24 174 / 470 us,
-// 200k of 2^28 53 / 91 us.
+// Measured, set / sort: 3M keys of 2^26 66 / 137 us, 20M of 2^24 174 / 470 us,
+// 200k of 2^28 53 / 91 us.  Sorts of one block are beaten from 6,000 keys on
+// where the set is at most 2 MB: 9,000 keys of 2^24 39 / 46 us, 5,000 38 / 36.
 constexpr uint64_t kKeysetSpacePerKey = 4096;
+constexpr uint64_t kKeysetMinKeys = 6000;
 
 bool sort_by_keyset(uint64_t n, int bits) {
-  return n > kRsSmall && 2 * bits <= kKeysetMaxBits && n >= (1ull << (2 * bits)) / kKeysetSpacePerKey;
+  return n > (2 * bits <= 24 ? kKeysetMinKeys : kRsSmall) && 2 * bits <= kKeysetMaxBits &&
+         n >= (1ull << (2 * bits)) / kKeysetSpacePerKey;
 }
 
 size_t sort_dev_scratch_bytes(uint64_t cap, uint64_t full_cap, int bits) {
