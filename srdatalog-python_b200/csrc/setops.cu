@@ -6,7 +6,7 @@
 // is known up front.  A first launch finds the merge-path split point of
 // every 2048-element output tile (one binary search per tile boundary); then
 // each block owns one output tile, stages both input slices in shared memory
-// with coalesced loads, merges 8 outputs per thread and writes the tile back
+// with coalesced loads, merges 16 outputs per thread and writes the tile back
 // coalesced.
 //
 // set_difference replaces thrust::set_difference on the zipped columns
@@ -25,8 +25,14 @@ static std::atomic<uint64_t> g_launches{0};
 void count_launches(int k) { g_launches.fetch_add((uint64_t)k, std::memory_order_relaxed); }
 uint64_t launches_total() { return g_launches.load(std::memory_order_relaxed); }
 
-constexpr int kMgThreads = 256;
-constexpr int kMgItems = 8;
+// A thread merges 16 outputs into registers, so the tile is merged in place and
+// its search is paid for by 16 keys instead of 8.  60M + 20M keys: 305 us, 338
+// with 256 threads, 8 outputs each and a second tile for the outputs, 347 with
+// 8 outputs in place, 322 with 16 and a second tile, 318 with 24 in place, 345
+// with 64 threads, 439 with 256; held to 48 or 40 registers (10 or 12 blocks
+// per SM instead of 8) 330 and 381.  Bound: shared memory accesses.
+constexpr int kMgThreads = 128;
+constexpr int kMgItems = 16;
 constexpr int kMgTile = kMgThreads * kMgItems;
 
 // Number of elements taken from `a` among the first `diag` merged outputs
@@ -84,17 +90,16 @@ __global__ void merge_split_kernel(const uint64_t* __restrict__ a, uint64_t na,
 }
 
 // Shared-memory index with one pad word per 16 keys: threads that walk the
-// tile 8 (or about 4) keys apart then hit different banks.
+// tile 16 keys apart then hit different banks.
 __device__ __forceinline__ int mg_pad(int p) { return p + (p >> 4); }
 constexpr int kMgPadded = kMgTile + kMgTile / 16;
 
-__global__ void __launch_bounds__(kMgThreads) merge_kernel(const uint64_t* __restrict__ a,
+__global__ void __launch_bounds__(kMgThreads, 8) merge_kernel(const uint64_t* __restrict__ a,
                                                            uint64_t na,
                                                            const uint64_t* __restrict__ b,
                                                            uint64_t nb,
                                                            uint64_t* __restrict__ out, MergeDev md) {
-  __shared__ uint64_t sin[kMgPadded];
-  __shared__ uint64_t sout[kMgPadded];
+  __shared__ uint64_t sin[kMgPadded + 1];  // inputs, then outputs; one word past the tile is read
   __shared__ uint64_t split[2];
   if (!merge_dev_sizes(md, na, nb)) return;
   const uint64_t total = na + nb;
@@ -111,10 +116,21 @@ __global__ void __launch_bounds__(kMgThreads) merge_kernel(const uint64_t* __res
     const uint64_t i0 = split[0], i1 = split[1];
     const uint64_t j0 = d0 - i0, j1 = d1 - i1;
     const int la = (int)(i1 - i0), lb = (int)(j1 - j0), lt = la + lb;
-    for (int k = threadIdx.x; k < lt; k += kMgThreads)
-      sin[mg_pad(k)] = k < la ? a[i0 + k] : b[j0 + k - la];
+    if (lt == kMgTile) {
+      uint64_t v[kMgItems];
+#pragma unroll
+      for (int q = 0; q < kMgItems; q++) {
+        const int k = threadIdx.x + q * kMgThreads;
+        v[q] = k < la ? a[i0 + k] : b[j0 + k - la];
+      }
+#pragma unroll
+      for (int q = 0; q < kMgItems; q++) sin[mg_pad(threadIdx.x + q * kMgThreads)] = v[q];
+    } else {
+      for (int k = threadIdx.x; k < lt; k += kMgThreads) sin[mg_pad(k)] = k < la ? a[i0 + k] : b[j0 + k - la];
+    }
     __syncthreads();
     const int ld = threadIdx.x * kMgItems;
+    uint64_t o[kMgItems];
     if (ld < lt) {
       int lo = ld > lb ? ld - lb : 0, hi = ld < la ? ld : la;
       while (lo < hi) {
@@ -122,24 +138,27 @@ __global__ void __launch_bounds__(kMgThreads) merge_kernel(const uint64_t* __res
         if (sin[mg_pad(mid)] <= sin[mg_pad(la + ld - 1 - mid)]) lo = mid + 1;
         else hi = mid;
       }
-      int i = lo, j = ld - lo;
-      uint64_t va = i < la ? sin[mg_pad(i)] : 0, vb = j < lb ? sin[mg_pad(la + j)] : 0;
+      // i: next of a, j: next of b (both as places in the tile).  A list that has
+      // run out leaves a value that the other's bound overrules.
+      int i = lo, j = la + ld - lo;
+      uint64_t va = sin[mg_pad(i)], vb = sin[mg_pad(j)];
 #pragma unroll
       for (int k = 0; k < kMgItems; k++) {
-        if (ld + k >= lt) break;
-        const bool take_a = (j >= lb) || (i < la && va <= vb);
-        sout[mg_pad(ld + k)] = take_a ? va : vb;
-        if (take_a) {
-          i++;
-          va = i < la ? sin[mg_pad(i)] : 0;
-        } else {
-          j++;
-          vb = j < lb ? sin[mg_pad(la + j)] : 0;
-        }
+        const bool take_a = (j >= lt) | ((i < la) & (va <= vb));
+        o[k] = take_a ? va : vb;
+        i += take_a;
+        j += !take_a;
+        const uint64_t next = sin[mg_pad(min(take_a ? i : j, kMgTile))];
+        va = take_a ? next : va;
+        vb = take_a ? vb : next;
       }
     }
+    __syncthreads();  // every thread has read its inputs
+#pragma unroll
+    for (int k = 0; k < kMgItems; k++)
+      if (ld + k < lt) sin[mg_pad(ld + k)] = o[k];
     __syncthreads();
-    for (int k = threadIdx.x; k < lt; k += kMgThreads) out[d0 + k] = sout[mg_pad(k)];
+    for (int k = threadIdx.x; k < lt; k += kMgThreads) out[d0 + k] = sin[mg_pad(k)];
     __syncthreads();  // the shared tiles are refilled for the next tile
   }
 }
