@@ -1083,21 +1083,32 @@ void Database::copy_rows(const uint64_t* keys, uint64_t n, int arity, uint32_t* 
     memcpy(dst, stage, n * row);
     return;
   }
-  const uint64_t per = kDumpPiece / row, pieces = (n + per - 1) / per;
+  uint64_t per = kDumpPiece / row, pieces = (n + per - 1) / per;
   const unsigned hw = std::thread::hardware_concurrency();
-  const int T = (int)std::min<uint64_t>({pieces, (uint64_t)kDumpThreads, std::max(1u, hw)});
+  int T = (int)std::min<uint64_t>({pieces, (uint64_t)kDumpThreads, std::max(1u, hw)});
   const size_t piece_bytes = std::min<uint64_t>(per, n) * row;
   DumpStage& shared = dump_stage();
   std::unique_lock<std::mutex> taken(shared.mu, std::try_to_lock);
   PinnedBuf& pinned = taken ? shared.buf : dump_buf_;
-  pinned.reserve(T * piece_bytes);
+  char* stages;
+  try {
+    pinned.reserve(T * piece_bytes);
+    stages = static_cast<char*>(pinned.p);
+  } catch (const Error&) {
+    // the host has no more memory to lock: the handle's own block, one thread
+    cudaGetLastError();
+    stages = reinterpret_cast<char*>(h_small_ + kSmallSlots);
+    per = kSmallRows / row & ~uint64_t(3);  // (whole 16-byte stores)
+    pieces = (n + per - 1) / per;
+    T = 1;
+  }
   std::vector<Error> errs((size_t)T, Error{0, ""});
   auto work = [&](int t) {
     cudaEvent_t ev = nullptr;
     try {
       SRDL_CUDA(cudaSetDevice(device_));
       SRDL_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-      char* stage = static_cast<char*>(pinned.p) + t * piece_bytes;
+      char* stage = stages + t * piece_bytes;
       for (uint64_t p = t; p < pieces; p += T) {
         const uint64_t r0 = p * per, cnt = std::min(per, n - r0);
         unpack_rows(L_, keys + r0, cnt, arity, stage);

@@ -24,18 +24,20 @@
 // overflow flag; kernels never write past a capacity).  One launch, one
 // host synchronisation.
 //
-// Where the key space is small (2^kKeysetMaxBits), NEW and FULL are bitmap sets
-// during the loop: the joins set the bits of the keys they derive, those FULL
-// lacks are listed as DELTA and added to FULL, and FULL is listed as a sorted
-// array once, after the last iteration -- no rule of a qualifying step reads it
-// before.  That takes the place of the sort, the set difference and the merge
-// of every iteration.  DELTA is written after the joins have read the one
-// before, so one buffer set is enough and the graph is WHILE (go) { iteration;
-// control }, half as long to capture and instantiate.  On overflow the failed iteration's inputs are
-// intact (they are the other buffer set): the host resumes from them on the
-// host path, and the next entry sizes the buffers from the larger counts
-// that path measures.  Results are those of the host path: the same
-// kernels, the same DELTA = unique(NEW) - FULL, FULL |= DELTA.
+// Where the key space is small (the rule is at `sets`), NEW and FULL are bitmap
+// sets during the loop: the joins set the bits of the keys they derive, those
+// FULL lacks are listed as DELTA and added to FULL, and FULL is listed as a
+// sorted array once, after the last iteration -- no rule of a qualifying step
+// reads it before.  That takes the place of the sort, the set difference and
+// the merge of every iteration.  DELTA is written after the joins have read the
+// one before, so one buffer set is enough and the graph is WHILE (go) {
+// iteration; control }, half as long to capture and instantiate.
+//
+// On overflow the failed iteration's inputs are intact (the other buffer set;
+// with bitmap sets DELTA and FULL have not been written): the host resumes from
+// them on the host path, and the next entry sizes the buffers from the larger
+// counts that path measures.  Results are those of the host path: the same
+// DELTA = unique(NEW) - FULL, FULL |= DELTA.
 #include <algorithm>
 #include <chrono>
 #include <cstdlib>
