@@ -473,12 +473,12 @@ def run_primitives(args, rank, world):
 
   ms = timed(sort)
   u = int(dn.item())
-  # packed key width k and the passes the library runs: read the input
-  # (8 B), write packed keys (k), P passes reading and writing k each, read
-  # the sorted keys once more (k) and write the distinct ones (8 B)
+  # packed key width k and the passes the library runs: the first reads the
+  # input (8 B) and writes packed keys (k), the others read and write k each,
+  # the sorted keys are read once more (k) and the distinct ones written (8 B)
   k = 4 if 2 * bits <= 32 else 8
-  passes = (2 * bits + 7) // 8  # the library's default widest digit is 8 bits
-  alg = n * (8 + k + passes * 2 * k + k) + 8 * u
+  passes = (2 * bits + 8) // 9  # the library's widest digit is 9 bits
+  alg = n * (8 + k + (passes - 1) * 2 * k + k) + 8 * u
   report('sort_unique', ms, alg, keys=n, unique=u, value_bits=bits, passes=passes,
          io_gbs=round(16 * n / ms / 1e6, 1))
   del scratch
