@@ -29,6 +29,11 @@ constexpr int kCpThreads = 256;
 constexpr int kCpWarps = kCpThreads / 32;
 constexpr int kCpItems = 8;
 constexpr int kCpTile = kCpThreads * kCpItems;
+// The mark pass of the set difference: 16 keys a thread pay for a thread's
+// search, and six blocks per SM (the shared memory's limit) fit one wave.  50M -
+// 30M keys 426 us, 467 with 256 threads of 8 keys and four blocks, 485 with six.
+constexpr int kDmThreads = 128;
+constexpr int kDmItems = kCpTile / kDmThreads;
 
 // Largest FULL, in multiples of the keys, that a set difference streams (its
 // merge path); past it every key is searched in FULL (its probe path).
@@ -170,7 +175,7 @@ void compact(const Launch& L, Sel sel, uint64_t n, uint64_t* d_total, Scratch& s
 // as (hi << bits) | lo and are expanded to (hi << 32) | lo on output.
 // PLAIN: the keys are whole (bits = 32) and distinct, known at compile time --
 // the standalone set difference, whose mark pass is bound by instructions: 50M
-// - 30M keys take 475 us, 525 when the pass treats them as the sort's.
+// - 30M keys took 504 us, 553 when the pass treated them as the sort's.
 template <typename K, bool PLAIN = false>
 struct DedupDiffSel {
   const K* a;
@@ -351,13 +356,13 @@ __device__ __forceinline__ void dm_fetch(const DedupDiffSel<K, PLAIN>& sel, unsi
                                          uint64_t i0, uint32_t la, uint64_t j0, uint32_t lf) {
   K* da = reinterpret_cast<K*>(buf);
   uint64_t* df = reinterpret_cast<uint64_t*>(buf + ((la * sizeof(K) + 7) & ~size_t(7)));
-  for (uint32_t k = threadIdx.x; k < la; k += kCpThreads) cp_async_small<sizeof(K)>(da + k, sel.a + i0 + k);
-  for (uint32_t k = threadIdx.x; k < lf; k += kCpThreads) cp_async_small<8>(df + k, sel.full + j0 + k);
+  for (uint32_t k = threadIdx.x; k < la; k += kDmThreads) cp_async_small<sizeof(K)>(da + k, sel.a + i0 + k);
+  for (uint32_t k = threadIdx.x; k < lf; k += kDmThreads) cp_async_small<8>(df + k, sel.full + j0 + k);
   asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
 
 template <typename K, bool PLAIN>
-__global__ void __launch_bounds__(kCpThreads) dm_mark_kernel(DedupDiffSel<K, PLAIN> sel, uint64_t na,
+__global__ void __launch_bounds__(kDmThreads) dm_mark_kernel(DedupDiffSel<K, PLAIN> sel, uint64_t na,
                                                              uint64_t tiles,
                                                              const uint64_t* __restrict__ split,
                                                              const uint64_t* __restrict__ hpos,
@@ -394,7 +399,7 @@ __global__ void __launch_bounds__(kCpThreads) dm_mark_kernel(DedupDiffSel<K, PLA
     const uint32_t la = (uint32_t)(i1 - i0), lf = (uint32_t)(j1 - j0);
     const uint64_t w0 = i0 / 32;
     const uint32_t nwords = la ? (uint32_t)((i1 - 1) / 32 - w0 + 1) : 0;
-    for (uint32_t k = threadIdx.x; k < nwords; k += kCpThreads) sbits[k] = 0;
+    for (uint32_t k = threadIdx.x; k < nwords; k += kDmThreads) sbits[k] = 0;
     // values just before the tile (for the first element of thread 0's run)
     const uint64_t edge_a = i0 > 0 ? sel.expand(sel.a[i0 - 1]) : 0;
     const uint64_t edge_f = j0 > 0 ? sel.full[j0 - 1] : 0;
@@ -410,7 +415,7 @@ __global__ void __launch_bounds__(kCpThreads) dm_mark_kernel(DedupDiffSel<K, PLA
     const K* sa = reinterpret_cast<const K*>(buf[cur]);
     const uint64_t* sf =
         reinterpret_cast<const uint64_t*>(buf[cur] + ((la * sizeof(K) + 7) & ~size_t(7)));
-    const uint32_t diag = threadIdx.x * kCpItems;
+    const uint32_t diag = threadIdx.x * kDmItems;
     if (diag < la + lf && la) {
       uint32_t lo = diag > lf ? diag - lf : 0, hi = diag < la ? diag : la;
       while (lo < hi) {
@@ -434,7 +439,7 @@ __global__ void __launch_bounds__(kCpThreads) dm_mark_kernel(DedupDiffSel<K, PLA
       bool again = !PLAIN & sel.dedup & has_p & (prev == x);          // x repeats the key before it
       const uint32_t sh = (uint32_t)(i0 - wbase * 32);                // i0 + ia - wbase * 32 < 64
 #pragma unroll
-      for (int q = 0; q < kCpItems; q++) {
+      for (int q = 0; q < kDmItems; q++) {
         const bool take_a = (jf >= lf) | ((ia < la) & (x < f));
         bool keep = take_a & (ia < la) & !known & !again;
         if (!PLAIN && keep && h1 > h0) {
@@ -463,7 +468,7 @@ __global__ void __launch_bounds__(kCpThreads) dm_mark_kernel(DedupDiffSel<K, PLA
       if (mask >> 32) atomicOr(&sbits[wbase + 1 - w0], (uint32_t)(mask >> 32));
     }
     __syncthreads();
-    for (uint32_t k = threadIdx.x; k < nwords; k += kCpThreads)
+    for (uint32_t k = threadIdx.x; k < nwords; k += kDmThreads)
       if (sbits[k]) atomicOr(&flags[w0 + k], sbits[k]);
     __syncthreads();
     if (tn >= tiles) break;
@@ -523,8 +528,8 @@ void compact_diff(const Launch& L, DedupDiffSel<K, PLAIN> sel, uint64_t n, uint6
     SRDL_CUDA(cudaMemsetAsync(flags, 0, cp_words(n) * 4, L.stream));
     dm_split_kernel<K, PLAIN><<<(unsigned)((mtiles + 1 + 255) / 256), 256, 0, L.stream>>>(sel, n, mtiles, split, mhpos,
                                                                                   nullptr, kPathAny);
-    const unsigned mgrid = (unsigned)std::min<uint64_t>(mtiles, (uint64_t)L.num_sms * 4);
-    dm_mark_kernel<K, PLAIN><<<mgrid, kCpThreads, 0, L.stream>>>(sel, n, mtiles, split, mhpos, flags, nullptr, kPathAny);
+    const unsigned mgrid = (unsigned)std::min<uint64_t>(mtiles, (uint64_t)L.num_sms * 6);
+    dm_mark_kernel<K, PLAIN><<<mgrid, kDmThreads, 0, L.stream>>>(sel, n, mtiles, split, mhpos, flags, nullptr, kPathAny);
     cp_count_kernel<K, PLAIN><<<nb, kCpThreads, 0, L.stream>>>(flags, n, chunk, counts, sel, nullptr, kPathAny);
     count_launches(3);
   } else {
@@ -568,8 +573,8 @@ void compact_diff_dev(const Launch& L, DedupDiffSel<K, PLAIN> sel, uint64_t cap,
   SRDL_CUDA(cudaMemsetAsync(flags, 0, cp_words(cap) * 4, L.stream));
   dm_split_kernel<K, PLAIN><<<(unsigned)((mtiles + 1 + 255) / 256), 256, 0, L.stream>>>(sel, cap, mtiles, split, nullptr,
                                                                                 d_n, kPathMerge);
-  const unsigned mgrid = (unsigned)std::min<uint64_t>(mtiles, (uint64_t)L.num_sms * 4);
-  dm_mark_kernel<K, PLAIN><<<mgrid, kCpThreads, 0, L.stream>>>(sel, cap, mtiles, split, nullptr, flags, d_n, kPathMerge);
+  const unsigned mgrid = (unsigned)std::min<uint64_t>(mtiles, (uint64_t)L.num_sms * 6);
+  dm_mark_kernel<K, PLAIN><<<mgrid, kDmThreads, 0, L.stream>>>(sel, cap, mtiles, split, nullptr, flags, d_n, kPathMerge);
   cp_count_kernel<K, PLAIN><<<nb, kCpThreads, 0, L.stream>>>(flags, cap, 0, counts, sel, d_n, kPathMerge);
   // probe path
   dd_probe_kernel<K, PLAIN><<<nb, kCpThreads, 0, L.stream>>>(sel, cap, 0, flags, counts, d_n, kPathProbe);
