@@ -281,8 +281,9 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
       {
         // the buffers below; leave the step to the host path rather than
         // take most of the free memory (the host path needs far less)
+        // (bitmap sets: FULL is listed into a buffer of its final size after the loop)
         const uint64_t need = lr.cap_delta * (sets ? 16 : 16 + 8 + 8) +
-                              (sets ? 2 * set_bytes
+                              (sets ? 2 * set_bytes + lr.cap_full * 8
                                     : lr.cap_new * 8 + lr.cap_full * 16 +
                                           sort_dev_scratch_bytes(lr.cap_new, lr.cap_full, bits_));
         size_t free_b = 0, total_b = 0;
@@ -650,6 +651,25 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
 
   // ---- the latest complete iteration becomes the host state
   const int q = (int)ctl.parity;
+  if (sets) {
+    // Room to list FULL, for every relation before any of them is replaced: an
+    // allocation refused here leaves the step to the host path, which starts
+    // again from the state the loop was entered with.
+    try {
+      for (size_t i = 0; i < X.rels.size(); i++) {
+        const uint64_t nf = cnt[i].n_full[q];
+        SRDL_REQUIRE(!opt_loop_cap_limit_ || nf <= X.rels[i].cap_full, kErrCapacity,
+                     "device loop: no room for FULL of " + X.rels[i].r->name);
+        X.rels[i].full[0] = DevBuf(std::max<uint64_t>(nf, 1) * 8, L_.stream);
+      }
+    } catch (const Error& e) {
+      if (e.code != kErrCapacity && e.code != kErrCuda) throw;
+      (void)cudaGetLastError();
+      loop_stats_.skipped++;
+      loop_stats_.last_error = e.msg;
+      return kLoopSkipped;
+    }
+  }
   for (size_t i = 0; i < X.rels.size(); i++) {
     LoopRel& lr = X.rels[i];
     Relation& r = *lr.r;
@@ -658,13 +678,10 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
     r.head = Index{};
     Index& f = r.v[kFull].idx[r.canonical];
     f.n = c.n_full[q];
-    if (sets) {
-      f.keys = DevBuf(std::max<uint64_t>(f.n, 1) * 8, L_.stream);
+    f.keys = std::move(lr.full[q]);  // (bitmap sets: q is 0)
+    if (sets)
       keyset_list(L_, lr.full_set.as<uint32_t>(), bits_, lr.set_counts.as<uint32_t>(), f.keys.as<uint64_t>(),
                   d_small_.as<uint64_t>());
-    } else {
-      f.keys = std::move(lr.full[q]);
-    }
     r.v[kDelta].clear();
     r.v[kNew].clear();
     Index& d = r.v[kDelta].idx[r.canonical];

@@ -90,6 +90,20 @@ def test_overflow_hands_iterations_back_to_the_host(cap, expected):
   assert rec_iterations(db)[0] == expected['tc_small']['iterations']
 
 
+def test_no_room_for_the_final_full():
+  '''The iterations of a long chain fit the loop, FULL's list after it does not
+  (a capacity of 16 times the limit stands for an allocation refused): nothing
+  has been replaced yet, so the host path runs the step from the state that the
+  loop was entered with.'''
+  e = np.stack([np.arange(600), np.arange(1, 601)], 1).astype(np.uint32)
+  db = run('tc', {'ArcInput': e}, cap=4096, repeat=2)
+  st = loop_stats(db)
+  assert st['skipped'] == 1 and st['overflows'] == 0 and 'FULL' in st['last_error'], st
+  same(db, run('tc', {'ArcInput': e}, loop=False), 'Path')
+  assert db.size('Path') == 600 * 601 // 2
+  assert rec_iterations(db) == [600]
+
+
 @pytest.mark.parametrize('max_iters', [1, 2, 3, 5, 9])
 def test_max_iters_on_the_device_loop(max_iters):
   e = W.uniform_edges(2000, 6000, 7)
