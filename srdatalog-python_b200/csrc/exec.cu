@@ -404,10 +404,14 @@ void Database::exec_pipeline(const Op& op, bool recursive, uint64_t iteration) {
       total = seg_owned(total, lv.seg, shard_world_, shard_rank_);
     }
     // the expand pass's own scratch, sized for this level's candidates
-    DevBuf xscr(join_expand_scratch_bytes(L_, total) + (w.poffs ? join_pivot_scratch_bytes(lv) : 0),
-                L_.stream);
-    Scratch xs{xscr.as<char>(), xscr.bytes(), 0};
+    DevBuf xscr;
+    Scratch xs;
+    auto take_scratch = [&](size_t bytes) {
+      xscr = DevBuf(bytes, L_.stream);
+      xs = Scratch{xscr.as<char>(), xscr.bytes(), 0};
+    };
     if (last) {
+      take_scratch(join_expand_scratch_bytes(L_, total) + (w.poffs ? join_pivot_scratch_bytes(lv) : 0));
       if (op.count) {
         lv.emit = kEmitCount;
         DevBuf gb, gc;
@@ -493,6 +497,14 @@ void Database::exec_pipeline(const Op& op, bool recursive, uint64_t iteration) {
       // candidate total as capacity and reads the true count itself.
       DevBuf count(8, L_.stream);
       if (!total) SRDL_CUDA(cudaMemsetAsync(count.as<void>(), 0, 8, L_.stream));
+      // (after the columns, so a memory limit that has no room for a small
+      // table's staged rows leaves out those and nothing else)
+      try {
+        take_scratch(join_expand_scratch_bytes(L_, total, true));
+      } catch (const Error& e) {
+        if (e.code != kErrCapacity) throw;
+        take_scratch(join_expand_scratch_bytes(L_, total));
+      }
       pid = prof_begin("join_expand_table");
       join_expand(L_, lv, cur, w, total, &next, nullptr, count.as<uint64_t>(), xs);
       prof_end(pid, 4.0 * total * std::max(1, lv.nsrc), (double)total);

@@ -896,15 +896,15 @@ static int jgrid(uint64_t n, const Launch& L) {
 // Most per-chunk counts the two-source column join keeps in its table modes.
 constexpr uint64_t kCj2MaxTableChunks = 1ull << 18;
 
-size_t join_expand_scratch_bytes(const Launch& L, uint64_t total) {
+size_t join_expand_scratch_bytes(const Launch& L, uint64_t total, bool staged) {
   // per-warp counts of the generic kernels' table modes, or per-chunk counts
   // of the two-source column join's (chunks of at least 64 candidates)
   const uint64_t warps = (uint64_t)jgrid(total, L) * (kJThreads / 32);
   const uint64_t chunks = std::min<uint64_t>(kCj2MaxTableChunks, (total + 63) / 64);
   const uint64_t n = std::max<uint64_t>(warps, chunks);
   // (+ the staged survivors of a small table)
-  const uint64_t staged = total <= kCj2StageTotal ? total * 8 + 256 : 0;
-  return 2 * ((n + 1) * 8 + 255) + scan_scratch_bytes(n) + 4096 + staged;
+  return 2 * ((n + 1) * 8 + 255) + scan_scratch_bytes(n) + 4096 +
+         (staged && total <= kCj2StageTotal ? total * 8 + 512 : 0);
 }
 
 // Resident blocks per SM of the two-source column-join kernel for a level
@@ -1298,7 +1298,7 @@ void join_expand(const Launch& L, const LevelSpec& lv, const Table& in, const Jo
       count_launches(1);
     } else {
       uint64_t* cc = s.take<uint64_t>(nchunks + 1);
-      if (total <= kCj2StageTotal) {
+      if (total <= kCj2StageTotal && s.used + total * 8 + 512 <= s.cap) {
         uint2* st = s.take<uint2>(total);
         SRDL_CJ2(kModeTableCount, q, cc, st);
         join_stage_kernel<<<(unsigned)((nchunks + kJThreads / 32 - 1) / (kJThreads / 32)), kJThreads, 0, L.stream>>>(

@@ -339,8 +339,10 @@ constexpr size_t kPivotSmemMax = 200 * 1024;
 // counted (emit count) via *d_out_n, which the caller zeroes for emit keys and
 // emit count (emit table sets it).  Output
 // capacity = total.  The scratch for a level of `total` candidates comes
-// from join_expand_scratch_bytes(L, total).
-size_t join_expand_scratch_bytes(const Launch& L, uint64_t total);
+// from join_expand_scratch_bytes(L, total); with `staged`, what a small table
+// takes to probe its candidates once is added (without that room it is
+// counted and written in two passes).
+size_t join_expand_scratch_bytes(const Launch& L, uint64_t total, bool staged = false);
 
 // Device loop: the candidate count is on the device (d_total, the count
 // pass's offs[rows]); `total` is then its capacity.  A count above the

@@ -425,6 +425,12 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
           const int bound = pp.levels[li + 1].n_in_slots;
           for (int c = 0; c < bound && c < kMaxSlots; c++)
             lvls[li].cols[c] = DevBuf(lvls[li].cap_total * 4, L_.stream);
+          // small tables: room for their staged rows, where a memory limit
+          // leaves it (and a megabyte for what the step still takes)
+          const size_t staged = join_expand_scratch_bytes(L_, lvls[li].cap_total, true);
+          const ArenaUse au = arena_use(L_.stream);
+          if (staged > lvls[li].xscr.bytes() && (!au.limit || au.in_use + 2 * staged + (1 << 20) <= au.limit))
+            lvls[li].xscr = DevBuf(staged, L_.stream);
         }
       } catch (const Error& e) {
         if (e.code != kErrCapacity && e.code != kErrCuda) throw;
