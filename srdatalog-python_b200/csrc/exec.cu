@@ -365,9 +365,6 @@ void Database::exec_pipeline(const Op& op, bool recursive, uint64_t iteration) {
   for (size_t li = 0; li < levels.size(); li++) {
     LevelSpec& lv = levels[li];
     const bool last = li + 1 == levels.size();
-    DevBuf wscr(join_work_scratch_bytes(cur.n), L_.stream);
-    Scratch s{wscr.as<char>(), wscr.bytes(), 0};
-    size_t pid = prof_begin("join_count");
     // the last level of a count-only rule: rows probing a long list of the
     // table's first column go to the pivot kernel (join.cu)
     lv.pivot_src = -1;
@@ -386,13 +383,27 @@ void Database::exec_pipeline(const Op& op, bool recursive, uint64_t iteration) {
         }
       }
     }
-    // (the totals land in page-locked memory: nothing is copied back)
-    JoinWork w = join_count(L_, lv, cur, s, d_small_.as<uint64_t>() + 2, h_small_ + 3, h_small_ + 6);
-    prof_end(pid, 8.0 * cur.n * (lv.n_in_slots + 3), (double)cur.n);
-    SRDL_CUDA(cudaStreamSynchronize(L_.stream));
-    uint64_t total = h_small_[3];
-    const uint64_t pivot_total = w.poffs ? h_small_[6] : 0;  // the pivot kernel's candidates
-    seen[li] = std::max(seen[li], total);
+    DevBuf wscr, xscr;  // the count pass's scratch; the expand pass's, sized for this level's candidates
+    Scratch s, xs;
+    auto take_scratch = [&](DevBuf& b, Scratch& sc, size_t bytes) {
+      b = DevBuf(bytes, L_.stream);
+      sc = Scratch{b.as<char>(), b.bytes(), 0};
+    };
+    JoinWork w;
+    uint64_t total = 0, pivot_total = 0;  // candidates of join_expand and of the pivot kernel
+    size_t pid;
+    auto count_level = [&] {
+      take_scratch(wscr, s, join_work_scratch_bytes(cur.n));
+      pid = prof_begin("join_count");
+      // (the totals land in page-locked memory: nothing is copied back)
+      w = join_count(L_, lv, cur, s, d_small_.as<uint64_t>() + 2, h_small_ + 3, h_small_ + 6);
+      prof_end(pid, 8.0 * cur.n * (lv.n_in_slots + 3), (double)cur.n);
+      SRDL_CUDA(cudaStreamSynchronize(L_.stream));
+      total = h_small_[3];
+      pivot_total = w.poffs ? h_small_[6] : 0;
+      seen[li] = std::max(seen[li], total);
+    };
+    count_level();
     if (sharded && op.shard == Op::Work && li == work_split) {
       // Deal this level's work items out in segments, kSegsPerShard per
       // shard, interleaved so every shard gets a share of each key range
@@ -403,15 +414,17 @@ void Database::exec_pipeline(const Op& op, bool recursive, uint64_t iteration) {
       lv.seg_rank = (uint32_t)shard_rank_;
       total = seg_owned(total, lv.seg, shard_world_, shard_rank_);
     }
-    // the expand pass's own scratch, sized for this level's candidates
-    DevBuf xscr;
-    Scratch xs;
-    auto take_scratch = [&](size_t bytes) {
-      xscr = DevBuf(bytes, L_.stream);
-      xs = Scratch{xscr.as<char>(), xscr.bytes(), 0};
-    };
     if (last) {
-      take_scratch(join_expand_scratch_bytes(L_, total) + (w.poffs ? join_pivot_scratch_bytes(lv) : 0));
+      try {
+        take_scratch(xscr, xs, join_expand_scratch_bytes(L_, total) + (w.poffs ? join_pivot_scratch_bytes(lv) : 0));
+      } catch (const Error& e) {
+        if (!w.poffs || e.code != kErrCapacity) throw;
+        // a memory limit without room for the pivot pass: its rows are counted with the others
+        lv.pivot_src = -1;
+        wscr.reset();
+        count_level();
+        take_scratch(xscr, xs, join_expand_scratch_bytes(L_, total));
+      }
       if (op.count) {
         lv.emit = kEmitCount;
         DevBuf gb, gc;
@@ -431,6 +444,7 @@ void Database::exec_pipeline(const Op& op, bool recursive, uint64_t iteration) {
           lv.grp_counts = gc.as<unsigned long long>();
         }
         pid = prof_begin("join_expand_count");
+        if (w.poffs) join_pivot_count(L_, lv, cur, w, d_small_.as<uint64_t>() + 2, xs);
         join_expand(L_, lv, cur, w, total, nullptr, nullptr, d_small_.as<uint64_t>() + 2, xs);
         if (lv.grp_counts) {
           std::vector<uint64_t> h(lv.n_groups);
@@ -500,10 +514,10 @@ void Database::exec_pipeline(const Op& op, bool recursive, uint64_t iteration) {
       // (after the columns, so a memory limit that has no room for a small
       // table's staged rows leaves out those and nothing else)
       try {
-        take_scratch(join_expand_scratch_bytes(L_, total, true));
+        take_scratch(xscr, xs, join_expand_scratch_bytes(L_, total, true));
       } catch (const Error& e) {
         if (e.code != kErrCapacity) throw;
-        take_scratch(join_expand_scratch_bytes(L_, total));
+        take_scratch(xscr, xs, join_expand_scratch_bytes(L_, total));
       }
       pid = prof_begin("join_expand_table");
       join_expand(L_, lv, cur, w, total, &next, nullptr, count.as<uint64_t>(), xs);

@@ -879,11 +879,11 @@ __global__ void __launch_bounds__(kJThreads) join_cart2_kernel(
 
 size_t join_work_scratch_bytes(uint64_t rows) {
   rows = rows ? rows : 1;
-  // (+ the chunk queues; the pivot rows' work, offsets and their scan)
+  // (+ the pivot rows' work, offsets and their scan)
   return ((rows * 8 + 255) & ~size_t(255)) + ((rows + 1) * 8 + 255) + ((rows + 255) & ~size_t(255)) +
          2 * ((rows * 4 + 255) & ~size_t(255)) + ((rows * 8 + 255) & ~size_t(255)) +
          scan_scratch_bytes(rows) + 1024 + ((rows * 8 + 255) & ~size_t(255)) + ((rows + 1) * 8 + 511) +
-         scan_scratch_bytes(rows) + 1024;
+         scan_scratch_bytes(rows) + 512;
 }
 
 static int jgrid(uint64_t n, const Launch& L) {
@@ -1224,8 +1224,8 @@ size_t join_pivot_scratch_bytes(const LevelSpec& lv) {
 
 // The pivot rows' count (count mode; w.poffs set): the runs of the long
 // lists' values, their pieces, then one block per SM over the pieces.
-static void join_pivot_count(const Launch& L, const LevelSpec& lv, const Table& in, const JoinWork& w,
-                             unsigned long long* d_out_n, Scratch& s) {
+void join_pivot_count(const Launch& L, const LevelSpec& lv, const Table& in, const JoinWork& w, uint64_t* d_out_n,
+                      Scratch& s) {
   const int ps = lv.pivot_src, ds = 1 - ps;
   const SrcSpec& P = lv.src[ps];
   const SrcSpec& D = lv.src[ds];
@@ -1249,7 +1249,8 @@ static void join_pivot_count(const Launch& L, const LevelSpec& lv, const Table& 
                                   d_runs, runs, pieces);
   exclusive_scan_u64(L, pieces, max_runs, piece_offs, s);
   join_pivot_count_kernel<<<L.num_sms, kPvThreads, smem, L.stream>>>(
-      dvals, w.poffs, w.beg, P.t.lo, P.t.dir, runs, piece_offs, d_runs, max_runs, pv_words(P.t.dir_n), q, d_out_n);
+      dvals, w.poffs, w.beg, P.t.lo, P.t.dir, runs, piece_offs, d_runs, max_runs, pv_words(P.t.dir_n), q,
+      reinterpret_cast<unsigned long long*>(d_out_n));
   SRDL_CUDA(cudaGetLastError());
   count_launches(2);
 }
@@ -1258,7 +1259,6 @@ void join_expand(const Launch& L, const LevelSpec& lv, const Table& in, const Jo
                  uint64_t total, Table* out_table, uint64_t* out_keys, uint64_t* d_out_n,
                  Scratch& s, const JoinDev* dev) {
   auto* cnt = reinterpret_cast<unsigned long long*>(d_out_n);
-  if (w.poffs && lv.emit == kEmitCount) join_pivot_count(L, lv, in, w, cnt, s);
   if (total == 0) return;
   const JoinDev jd = dev ? *dev : JoinDev{};
   const int g = jgrid(total, L);

@@ -328,8 +328,11 @@ JoinWork join_count(const Launch& L, const LevelSpec& lv, const Table& in, Scrat
 // directory of dir_n entries covers; levels that need more than kPivotSmemMax
 // keep the cj2 kernel.
 size_t join_pivot_smem_bytes(uint32_t dir_n);
-// Scratch the pivot pass adds to a level's expand scratch.
+// Scratch of the pivot pass, and the pass: adds the pivot rows' survivors to
+// *d_out_n (emit count; join_expand counts the other rows).
 size_t join_pivot_scratch_bytes(const LevelSpec& lv);
+void join_pivot_count(const Launch& L, const LevelSpec& lv, const Table& in, const JoinWork& w, uint64_t* d_out_n,
+                      Scratch& s);
 constexpr size_t kPivotSmemMax = 200 * 1024;
 
 // Pass 2: expands `total` work items (all of the count pass's items, or

@@ -130,3 +130,27 @@ def test_pivot_hub_of_many_pieces():
       db.run()
       counts.append(db.count('TriangleJoin'))
   assert counts[0] == counts[1] == oracle.triangle_count(e)
+
+
+@pytest.mark.parametrize('pivot_min', [1, 20])
+def test_pivot_rows_under_a_memory_limit(pivot_min):
+  '''A limit that the run fits under without the pivot rows' scratch.'''
+  e = W.rmat_edges(14, 350_000, seed=9)
+  want = oracle.triangle_count(e)
+  with native.Database(load_plan('triangle')) as db:
+    db.set_option('bitmap_mb', 0)
+    db.set_option('pivot_min', 0)
+    db.load_rows('KnowsInput', e)
+    db.set_option('mem_limit_mb', 1 << 12)
+    db.run()
+    limit = -(-db.mem_stats()['peak'] // (1 << 20))
+    db.set_option('mem_limit_mb', limit)
+    db.run()
+    assert db.count('TriangleJoin') == want
+    db.set_option('pivot_min', pivot_min)
+    db.run()
+    assert db.count('TriangleJoin') == want
+    assert db.mem_stats()['peak'] <= limit << 20
+    db.set_option('mem_limit_mb', 0)
+    db.run()
+    assert db.count('TriangleJoin') == want
