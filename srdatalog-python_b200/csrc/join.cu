@@ -34,8 +34,11 @@ namespace srdl {
 
 constexpr int kJThreads = 256;
 constexpr uint32_t kNoPair = 0xffffffffu;
-// Pivot rows: the driving list is at most this many times the pivot's list.
+// Pivot rows: the driving list is at most this many times the pivot's list and
+// has at least so many values (a row costs the pivot kernel its staging whatever
+// its length).
 constexpr uint32_t kPvRatio = 3;
+constexpr uint32_t kPvMinDrive = 16;
 
 // Position of the pair (a, b) in a pair index (a binary view whose row
 // positions number the pairs), or kNoPair.
@@ -157,11 +160,11 @@ __global__ void __launch_bounds__(SCAN ? SCAN : kJThreads, SCAN ? 1 : 8) join_co
       int bd = n1 < n0 ? 1 : 0;
       // a pivot row: the pivot source's list is long enough to be held as a
       // bitmap by the pivot kernel, and the other list, which then drives, is
-      // at most kPvRatio times as long
+      // neither a few values nor more than kPvRatio times as long
       bool piv = false;
       if (pwork) {
         const uint32_t np = lv.pivot_src == 0 ? n0 : n1, nd = lv.pivot_src == 0 ? n1 : n0;
-        piv = np >= lv.pivot_min && nd <= (uint64_t)kPvRatio * np;
+        piv = np >= lv.pivot_min && nd >= kPvMinDrive && nd <= (uint64_t)kPvRatio * np;
         if (piv) bd = 1 - lv.pivot_src;
       }
       const uint32_t* dv = bd ? v1 : v0;
@@ -952,12 +955,21 @@ static int cj2_blocks_per_sm(bool seg, int emit) {
 // uniform in single bits (R-MAT's are 0 three times out of four), and without
 // the fold a lookup took eight wavefronts.  1,024 rows at a time are staged in
 // shared memory, one per thread: the thread tests the up to six candidates that
-// share a 16-byte quad with another row itself, the whole quads between them are
-// numbered by one block scan, and warps take 512 quads at a time, so short rows
-// and a hub's long ones cost the same per candidate and no lane idles.  A lane
-// finds its first quad's row by binary search in shared memory and steps forward
-// from there, four loads in flight.  The next piece is looked up while the
-// current one is counted.
+// share a 16-byte quad with another row itself, one block scan numbers the whole
+// quads between them and the rows that have any, and warps take 512 quads at a
+// time, so short rows and a hub's long ones cost the same per candidate and no
+// lane idles.  A lane finds its first quad's row by binary search in shared
+// memory and steps forward from there, four loads in flight.  The next piece is
+// looked up while the current one is counted.
+//
+// Rows of fewer than 16 driving values stay with the other rows, and staged rows
+// without a whole quad are not stepped over: a hub of a sparse power-law graph
+// has most of its candidates in a few rows among tens of thousands that have a
+// handful each, and one block staged and stepped over them all (1M nodes, 4M
+// edges, ids distributed as the cube of a uniform number: 1.21 ms for the level,
+// 0.56 now, 0.38 without this kernel; the whole run 2.15, 1.49 and 1.45 ms).  A
+// line at 8 or 32 values: 0.68 and 0.49 ms there, -0.04 and +0.11 ms on the
+// triangle below.
 //
 // R-MAT scale 20 triangle (3.0e9 candidates if the shorter list always drives):
 // the level took 7.64 ms on join_cj2_kernel alone and takes 5.08 ms with the
@@ -1033,7 +1045,7 @@ __global__ void __launch_bounds__(kPvThreads, 1) join_pivot_count_kernel(
   };
   __shared__ Piece pc[2];
   __shared__ unsigned int s_next;         // next quads to take
-  __shared__ uint32_t s_inc[kPvThreads];  // staged rows: quads up to and including the row's
+  __shared__ uint32_t s_inc[kPvThreads];  // staged rows with whole quads: quads up to and including the row's
   __shared__ uint32_t s_base[kPvThreads]; // s_base + (quad number) = quad of dvals
   __shared__ uint32_t scan_sh[kPvThreads / 32 + 1];
   __shared__ unsigned long long s_sum[kPvThreads / 32];
@@ -1104,9 +1116,17 @@ __global__ void __launch_bounds__(kPvThreads, 1) join_pivot_count_kernel(
       const uint32_t qa = (b + 3) / 4, qb = e / 4;
       const uint32_t m = qb > qa ? qb - qa : 0;
       uint32_t quads;
-      const uint32_t ex = block_excl_scan(m, scan_sh, &quads);
-      s_inc[threadIdx.x] = ex + m;
-      s_base[threadIdx.x] = qa - ex;
+      s_inc[threadIdx.x] = 0xffffffffu;  // (past the last staged row: never stepped over)
+      // (one scan numbers the rows that have whole quads, from bit 20 on, and
+      // the quads: at most 2^17 of a piece)
+      uint32_t ex = block_excl_scan(m | (m ? 1u << 20 : 0u), scan_sh, &quads);
+      const uint32_t at = ex >> 20;
+      ex &= (1u << 20) - 1;
+      quads &= (1u << 20) - 1;
+      if (m) {
+        s_inc[at] = ex + m;
+        s_base[at] = qa - ex;
+      }
       {
         const uint32_t h1 = 4 * qa < e ? 4 * qa : e, t0 = 4 * qb > h1 ? 4 * qb : h1;
         uint32_t n = 0;

@@ -115,6 +115,23 @@ def test_pivot_rows_of_every_length(scale, draws, pivot_min):
     assert db.count('TriangleJoin') == oracle.triangle_count(e)
 
 
+@pytest.mark.parametrize('n', [1500, 5000])
+def test_pivot_hub_of_short_rows(n):
+  '''A hub's rows on both sides of the shortest list that is staged (16), some
+  without a whole quad and some empty, more of them than a block stages at once.'''
+  i = np.arange(1, n, dtype=np.int64)
+  own = np.concatenate([np.stack([i, i + d], 1)[(i % 41 >= d) & (i + d < n)] for d in range(1, 41)])
+  hub = np.stack([np.zeros(n - 1, np.int64), i], 1)
+  e = np.concatenate([hub, own]).astype(np.uint32)
+  want = oracle.triangle_count(e)
+  for pm in (1, 16, 1000):
+    with native.Database(load_plan('triangle')) as db:
+      db.set_option('pivot_min', pm)
+      db.load_rows('KnowsInput', e)
+      db.run()
+      assert db.count('TriangleJoin') == want
+
+
 def test_pivot_hub_of_many_pieces():
   '''One value whose rows make several million candidates.'''
   hub = np.stack([np.zeros(5000, np.uint32), np.arange(1, 5001, dtype=np.uint32)], 1)
