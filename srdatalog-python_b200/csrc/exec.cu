@@ -443,8 +443,13 @@ void Database::exec_pipeline(const Op& op, bool recursive, uint64_t iteration) {
           lv.n_groups = (uint32_t)ng;
           lv.grp_counts = gc.as<unsigned long long>();
         }
+        if (w.poffs) {
+          // per candidate its value (4 B), looked up in shared memory
+          pid = prof_begin("join_pivot_count");
+          join_pivot_count(L_, lv, cur, w, d_small_.as<uint64_t>() + 2, xs);
+          prof_end(pid, 4.0 * pivot_total, (double)pivot_total);
+        }
         pid = prof_begin("join_expand_count");
-        if (w.poffs) join_pivot_count(L_, lv, cur, w, d_small_.as<uint64_t>() + 2, xs);
         join_expand(L_, lv, cur, w, total, nullptr, nullptr, d_small_.as<uint64_t>() + 2, xs);
         if (lv.grp_counts) {
           std::vector<uint64_t> h(lv.n_groups);
@@ -456,7 +461,7 @@ void Database::exec_pipeline(const Op& op, bool recursive, uint64_t iteration) {
           for (size_t g = 0; g < h.size(); g++) acc[g] += h[g];
         }
         // per candidate: its value (4 B) and one probed word of each other list (4 B)
-        prof_end(pid, 4.0 * (total + pivot_total) * std::max(1, lv.nsrc), (double)(total + pivot_total));
+        prof_end(pid, 4.0 * total * std::max(1, lv.nsrc), (double)total);
         counts_[op.rule] += read_scalar(2);
       } else {
         lv.emit = kEmitKeys;

@@ -63,6 +63,9 @@ int value_bits(uint32_t max_value);
 // Counting passes the sort makes over keys of two dom_bits halves.
 int radix_passes(const Launch& L, int dom_bits);
 
+// Sorts of up to this many keys are one launch of one block.
+constexpr uint64_t kSortSmall = 16384;
+
 // Scratch needed by sort_dedup for n input keys.
 size_t sort_scratch_bytes(uint64_t n, int dom_bits);
 

@@ -89,7 +89,7 @@ __global__ void loop_ctrl_kernel(LoopCtl* ctl, LoopCounts* cnt, int nrel, int p,
       // emitted keys, the sort with its fused difference, the merge and
       // the delta's trie view -- the bytes the host path charges for them
       if (ks)
-        ctl->alg_bytes += 8.0 * nn + passes * 2.0 * ks * nn + 8.0 * nn + 2.0 * ks * nn + 8.0 * nd +
+        ctl->alg_bytes += 8.0 * nn + passes * 2.0 * ks * nn + 8.0 * nn + 8.0 * nd +
                           8.0 * nn + 16.0 * (nf + nd) + 16.0 * nd;
       else
         ctl->alg_bytes += 8.0 * nn + 2.0 * set_bytes + 8.0 * nd + 16.0 * nd;

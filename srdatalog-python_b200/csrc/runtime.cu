@@ -751,15 +751,15 @@ void Database::sort_into(Index& out, const uint64_t* in, uint64_t n, bool swap, 
             (unsigned long long)(full ? full->n : 0), (unsigned long long)(hd ? head->n : 0),
             (unsigned long long)out.n);
   if (pid != (size_t)-1) {
-    // Algorithmic bytes: each counting pass reads and writes the packed
-    // keys once; packing reads the input; the dedup pass reads the sorted
-    // keys and writes the distinct ones (plus one probe word per key into
-    // FULL when the delta is fused).
-    // A bitmap set reads the keys (and FULL) once and writes the distinct ones.
-    const double ks = by_set ? 0 : 2 * kb <= 32 ? 4 : 8;
-    const double passes = radix_passes(L_, kb);
-    kev_[pid].bytes = passes * 2 * ks * n + 8.0 * n + ks * n + ks * n + 8.0 * out.n +
-                      (diff ? 8.0 * n : 0);
+    // Algorithmic bytes: the keys are read and the distinct ones written.  A
+    // bitmap set is cleared and listed and reads FULL and HEAD besides; the
+    // others probe one word of FULL per key, and the counting passes write and
+    // read the packed keys once each (the first packs, the last read is the
+    // dedup pass's), which one block does in shared memory.
+    const double known = (double)(full ? full->n : 0) + (double)(hd ? head->n : 0);
+    const double packed = by_set || n <= kSortSmall ? 0 : radix_passes(L_, kb) * 2.0 * (2 * kb <= 32 ? 4 : 8);
+    kev_[pid].bytes = (8.0 + packed) * n + 8.0 * out.n +
+                      (by_set ? 8.0 * keyset_words(kb) + 8.0 * known : diff ? 8.0 * n : 0);
   }
 }
 

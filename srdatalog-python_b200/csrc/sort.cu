@@ -356,6 +356,7 @@ __global__ void __launch_bounds__(kRsThreads, 2) rs_scatter(const void* __restri
 constexpr int kRsSmallThreads = 1024;
 constexpr int kRsSmallWarps = kRsSmallThreads / 32;
 constexpr uint64_t kRsSmall = (uint64_t)kRsSmallThreads * kRsItems;
+static_assert(kRsSmall == kSortSmall, "one thread per kRsItems keys");
 constexpr int kRsSmallBits = 8;
 constexpr int kRsSmallPairs = 1 << (kRsSmallBits - 1);
 

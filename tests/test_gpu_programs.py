@@ -433,6 +433,25 @@ def test_tuning_options_keep_results(expected, radix_bits, jbpsm):
   assert t.count('TriangleJoin') == expected['triangle_rmat14']['count']
 
 
+@pytest.mark.parametrize('bits,m,keys', [(17, 9000, 'one block'), (13, 90_000, 'set'), (15, 60_000, 'passes'),
+                                         (18, 60_000, 'passes')])
+def test_sort_bytes(bits, m, keys):
+  '''The bytes charged to the sort family are those its path moves: keys in,
+  distinct keys out, a set's bits twice, or the packed keys twice per pass.'''
+  e = W.uniform_edges(1 << bits, m, 3)
+  e[0] = (1 << bits) - 1, 0
+  e = np.unique(e, axis=0)
+  db = native.Database(load_plan('triangle'))
+  db.set_profiling(True)
+  db.load_rows('KnowsInput', np.concatenate([e, e[: m // 3]]))
+  db.run()
+  k = db.stats()['kernels']['sort_dedup']
+  n, out = e.shape[0] + m // 3, e.shape[0]
+  extra = {'one block': 0, 'set': 2 * (1 << 2 * bits) // 8,
+           'passes': -(-2 * bits // 9) * 2 * (4 if bits <= 16 else 8) * n}[keys]
+  assert k['scopes'] == 1 and k['bytes'] == pytest.approx(8 * n + extra + 8 * out, rel=1e-5)  # (six digits printed)
+
+
 @pytest.mark.parametrize('n,m,seed', [(60, 400, 0), (3000, 60_000, 1)])
 def test_lsqb_q3_materialised_arity3(n, m, seed):
   '''LSQB Q3: a materialised arity-3 relation (packed keys), nine atoms, a
