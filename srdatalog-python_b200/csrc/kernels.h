@@ -69,8 +69,9 @@ constexpr uint64_t kSortSmall = 16384;
 // Scratch needed by sort_dedup for n input keys.
 size_t sort_scratch_bytes(uint64_t n, int dom_bits);
 
-// Whether sort_dedup takes n keys as a bitmap set, given scratch for it.
-bool sort_by_keyset(uint64_t n, int dom_bits);
+// Whether sort_dedup takes n keys as a bitmap set, given scratch for it, when
+// n_known keys (FULL and HEAD) are taken out.
+bool sort_by_keyset(uint64_t n, int dom_bits, uint64_t n_known = 0);
 
 // Radix-sorts n uint64 keys (both 32-bit halves < 2^dom_bits; halves
 // swapped first when `swap` is set) and writes the distinct keys, in

@@ -734,12 +734,13 @@ void Database::sort_into(Index& out, const uint64_t* in, uint64_t n, bool swap, 
   // (room for a bitmap set where the sort would take one, unless the run's
   // memory is limited: up to 32 MB more than the counting passes need)
   size_t sb = sort_scratch_bytes(n, kb);
-  if (!opt_mem_limit_ && sort_by_keyset(n, kb)) sb = std::max(sb, keyset_scratch_bytes(L_, kb));
+  const bool hd = head && head->n;
+  const uint64_t known = (full ? full->n : 0) + (hd ? head->n : 0);
+  if (!opt_mem_limit_ && sort_by_keyset(n, kb, known)) sb = std::max(sb, keyset_scratch_bytes(L_, kb));
   DevBuf scratch(sb, L_.stream);
   Scratch s{scratch.as<char>(), scratch.bytes(), 0};
-  const bool by_set = sort_by_keyset(n, kb) && keyset_scratch_bytes(L_, kb) <= sb;
-  const bool hd = head && head->n;
-  const bool diff = (full && full->n) || hd;
+  const bool by_set = sort_by_keyset(n, kb, known) && keyset_scratch_bytes(L_, kb) <= sb;
+  const bool diff = known > 0;
   size_t pid = prof_begin(diff ? "sort_dedup_diff" : "sort_dedup");
   sort_dedup(L_, in, n, kb, swap, full && full->n ? full->keys.as<uint64_t>() : nullptr,
              full ? full->n : 0, out.keys.as<uint64_t>(), d_small_.as<uint64_t>(), s,
@@ -756,7 +757,6 @@ void Database::sort_into(Index& out, const uint64_t* in, uint64_t n, bool swap, 
     // others probe one word of FULL per key, and the counting passes write and
     // read the packed keys once each (the first packs, the last read is the
     // dedup pass's), which one block does in shared memory.
-    const double known = (double)(full ? full->n : 0) + (double)(hd ? head->n : 0);
     const double packed = by_set || n <= kSortSmall ? 0 : radix_passes(L_, kb) * 2.0 * (2 * kb <= 32 ? 4 : 8);
     kev_[pid].bytes = (8.0 + packed) * n + 8.0 * out.n +
                       (by_set ? 8.0 * keyset_words(kb) + 8.0 * known : diff ? 8.0 * n : 0);

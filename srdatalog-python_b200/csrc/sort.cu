@@ -570,12 +570,17 @@ static inline bool use32(int bits) { return 2 * bits <= 32; }
 // Measured, set / sort: 3M keys of 2^26 66 / 137 us, 20M of 2^24 174 / 470 us,
 // 200k of 2^28 53 / 91 us.  Sorts of one block are beaten from 6,000 keys on
 // where the set is at most 2 MB: 9,000 keys of 2^24 39 / 46 us, 5,000 38 / 36.
+// FULL and HEAD are read whole to take their keys out of a set, and searched once
+// per key otherwise, so they are compared with the keys.  70k keys of 2^26 against
+// 10M of FULL 59 / 77 us and against 30M 140 / 81; 1M against 30M 146 / 152 and,
+// of 2^28, against 100M 406 / 224; 4M against 100M 426 / 452.
 constexpr uint64_t kKeysetSpacePerKey = 4096;
 constexpr uint64_t kKeysetMinKeys = 6000;
+constexpr uint64_t kKeysetKnown = 12u << 20, kKeysetKnownPerKey = 16;
 
-bool sort_by_keyset(uint64_t n, int bits) {
+bool sort_by_keyset(uint64_t n, int bits, uint64_t n_known) {
   return n > (2 * bits <= 24 ? kKeysetMinKeys : kRsSmall) && 2 * bits <= kKeysetMaxBits &&
-         n >= (1ull << (2 * bits)) / kKeysetSpacePerKey;
+         n >= (1ull << (2 * bits)) / kKeysetSpacePerKey && n_known <= kKeysetKnown + kKeysetKnownPerKey * n;
 }
 
 size_t sort_dev_scratch_bytes(uint64_t cap, uint64_t full_cap, int bits) {
@@ -637,7 +642,7 @@ void sort_dedup(const Launch& L, const uint64_t* in, uint64_t n, int bits, bool 
     return;
   }
   SRDL_REQUIRE(n < (1ull << 32), kErrCapacity, "sort: more than 2^32-1 rows in one index");
-  if (sort_by_keyset(n, bits) && s.used + keyset_scratch_bytes(L, bits) <= s.cap) {
+  if (sort_by_keyset(n, bits, (full ? n_full : 0) + (head ? n_head : 0)) && s.used + keyset_scratch_bytes(L, bits) <= s.cap) {
     keyset_dedup(L, in, n, bits, swap, full, full ? n_full : 0, head, n_head, out, d_nout, s);
     return;
   }

@@ -452,6 +452,21 @@ def test_sort_bytes(bits, m, keys):
   assert k['scopes'] == 1 and k['bytes'] == pytest.approx(8 * n + extra + 8 * out, rel=1e-5)  # (six digits printed)
 
 
+def test_few_keys_against_a_large_full():
+  '''A late iteration's NEW does not read all of FULL: 72,000 keys of 26 bits,
+  14.4M in FULL.'''
+  a, b = np.meshgrid(np.arange(3600), np.arange(4000, 8000), indexing='ij')
+  c = np.stack([np.arange(8000, 8018), np.arange(18) * 200], 1)   # new sources of 18 of the rows
+  e = np.concatenate([np.stack([a.ravel(), b.ravel()], 1), c, [[8191, 8191]]]).astype(np.uint32)
+  db = native.Database(load_plan('tc'))
+  db.set_option('device_loop', 0)
+  db.set_profiling(True)
+  db.load_rows('ArcInput', e)
+  db.run()
+  assert db.size('Path') == e.shape[0] + 18 * 4000
+  assert db.stats()['kernels']['sort_dedup_diff']['bytes'] < 8 * e.shape[0] / 10
+
+
 @pytest.mark.parametrize('n,m,seed', [(60, 400, 0), (3000, 60_000, 1)])
 def test_lsqb_q3_materialised_arity3(n, m, seed):
   '''LSQB Q3: a materialised arity-3 relation (packed keys), nine atoms, a
