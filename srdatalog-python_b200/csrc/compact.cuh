@@ -35,12 +35,16 @@ constexpr int kCpTile = kCpThreads * kCpItems;
 constexpr int kDmThreads = 128;
 constexpr int kDmItems = kCpTile / kDmThreads;
 
-// Largest FULL, in multiples of the keys, that a set difference streams (its
-// merge path); past it every key is searched in FULL (its probe path).
-// Measured, merge / probe: 1M keys against 4M 69 / 55 us and against 8M 85 / 55
-// us, 10M against 30M 267 / 271 us; but 10M against 15M 193 / 247 us and 50M
-// against 30M 549 / 957 us.
-constexpr uint64_t kDmMaxFullRatio = 2;
+// Whether a set difference streams FULL (its merge path) or searches every key in
+// it (its probe path).  Streaming costs both sides, a search one key, and few keys
+// leave a merge's launches waiting on one another: the line is at 4.5 times the
+// keys less 7M.  Merge / probe, us: 1M keys against 1M 40 / 33; 2M against 2M 50 /
+// 45 and against 600k 39 / 41; 4M against 8M 78 / 85, 12M 96 / 91 and 16M 107 /
+// 93; 10M against 30M 194 / 212 and 40M 222 / 225; 20M against 80M 398 / 435 and
+// 100M 465 / 444; 50M against 25M 458 / 872 and 200M 953 / 1003.
+__host__ __device__ inline bool dm_merges(uint64_t n, uint64_t n_full) {
+  return 2 * (n_full + 7000000) <= 9 * n;
+}
 
 // Grid shape for n elements: every block owns `chunk` elements (a multiple
 // of the tile), at most 8 blocks per SM, no empty blocks.
@@ -64,9 +68,9 @@ inline uint64_t cp_words(uint64_t n) { return (n + 31) / 32; }
 inline size_t cp_scratch_bytes(uint64_t n) {
   // flag words + per-block counts (blocks <= 8 per SM; 256 SMs bound), and for
   // the set difference the merge-path cuts and HEAD positions of every tile
-  // boundary (FULL at most kDmMaxFullRatio times the keys there), each piece
-  // padded to 256 bytes, plus alignment slack for the region itself
-  const uint64_t mtiles = ((kDmMaxFullRatio + 1) * n + kCpTile - 1) / kCpTile + 2;
+  // boundary (FULL at most 4.5 times the keys there), each piece padded to 256
+  // bytes, plus alignment slack for the region itself
+  const uint64_t mtiles = (n * 11 / 2 + kCpTile - 1) / kCpTile + 2;
   return ((cp_words(n) * 4 + 255) & ~uint64_t(255)) + (size_t)(256 * 8 + 1) * 4 + 3 * 256 +
          2 * ((mtiles * 8 + 255) & ~uint64_t(255)) + 256;
 }
@@ -216,8 +220,7 @@ enum DiffPath : int { kPathAny = 0, kPathMerge = 1, kPathProbe = 2 };
 template <typename K, bool PLAIN>
 __device__ __forceinline__ bool diff_path_runs(int path, const DedupDiffSel<K, PLAIN>& sel, uint64_t n) {
   if (path == kPathAny) return true;
-  const bool merge = sel.n_full <= kDmMaxFullRatio * n;
-  return (path == kPathMerge) == merge;
+  return (path == kPathMerge) == dm_merges(n, sel.n_full);
 }
 
 // lower_bound of kDdKeys keys of one lane in a[0..n) (n > 0): the halvings are
@@ -503,8 +506,8 @@ static __global__ void __launch_bounds__(kCpThreads) cp_count_kernel(const uint3
   if (threadIdx.x == 0) blk_counts[blockIdx.x] = tot;
 }
 
-// compact() for DedupDiffSel with a FULL array: merge path when FULL is not
-// much larger than the keys, one search per key otherwise.
+// compact() for DedupDiffSel with a FULL array: merge path or one search per key
+// (dm_merges).
 template <typename K, bool PLAIN>
 void compact_diff(const Launch& L, DedupDiffSel<K, PLAIN> sel, uint64_t n, uint64_t* d_total, Scratch& s) {
   if (!sel.head || sel.n_head == 0) {
@@ -520,7 +523,7 @@ void compact_diff(const Launch& L, DedupDiffSel<K, PLAIN> sel, uint64_t n, uint6
   const int nb = cp_blocks(n, chunk);
   uint32_t* flags = s.take<uint32_t>(cp_words(n));
   uint32_t* counts = s.take<uint32_t>(nb);
-  if (sel.n_full && sel.n_full <= kDmMaxFullRatio * n) {
+  if (sel.n_full && dm_merges(n, sel.n_full)) {
     const uint64_t mtiles = (n + sel.n_full + kCpTile - 1) / kCpTile;
     SRDL_REQUIRE(mtiles < (1ull << 31), kErrCapacity, "set difference: too many rows");
     uint64_t* split = s.take<uint64_t>(mtiles + 1);

@@ -55,7 +55,10 @@ def test_sort_unique_one_digit(n):
 
 
 @pytest.mark.parametrize('na,nb', [(1, 4), (2047, 2049), (2048, 2048), (31, 6000), (4096, 4096 * 16),
-                                   (4096, 4096 * 16 + 1), (20_481, 700_000), (1_300_000, 2)])
+                                   (4096, 4096 * 16 + 1), (20_481, 700_000), (1_300_000, 2),
+                                   # both sides of the line between streaming FULL and searching it
+                                   (1_555_556, 1), (1_555_556, 3), (2_000_000, 2_000_000), (2_000_000, 2_000_001),
+                                   (2_043_904, 4097), (2_043_905, 2047), (3_000_017, 6_500_076)])
 def test_set_difference_tile_edges(na, nb):
   rng = np.random.default_rng(na + nb)
   u = np.unique(np.concatenate([keys_with_bits(rng, na + nb, 32), np.array([0, TOP], np.uint64)]))
