@@ -634,6 +634,20 @@ static void sort_dedup_t(const Launch& L, const uint64_t* in, uint64_t n, int bi
   else compact_diff(L, sel, n, d_nout, s);
 }
 
+// One block and bitmap sets take less scratch than counting passes: a region that
+// two copies of the packed keys and the counters of 8-bit passes over 2,048-key
+// tiles do not fit in is refused whichever path the keys take.
+static void require_room(const Launch& L, uint64_t n, int bits, Scratch s) {
+  const size_t ks = use32(bits) ? 4 : 8;
+  const int nb = cp_blocks(n, cp_chunk(n, L.num_sms));
+  s.take<char>(n * ks);
+  s.take<char>(n * ks);
+  s.take<uint32_t>((size_t)256 * nb);
+  s.take<uint32_t>(256);
+  s.take<uint32_t>(cp_words(n));
+  s.take<uint32_t>(nb);
+}
+
 void sort_dedup(const Launch& L, const uint64_t* in, uint64_t n, int bits, bool swap,
                 const uint64_t* full, uint64_t n_full, uint64_t* out, uint64_t* d_nout,
                 Scratch& s, const uint64_t* head, uint64_t n_head) {
@@ -642,6 +656,7 @@ void sort_dedup(const Launch& L, const uint64_t* in, uint64_t n, int bits, bool 
     return;
   }
   SRDL_REQUIRE(n < (1ull << 32), kErrCapacity, "sort: more than 2^32-1 rows in one index");
+  require_room(L, n, bits, s);
   if (sort_by_keyset(n, bits, (full ? n_full : 0) + (head ? n_head : 0)) && s.used + keyset_scratch_bytes(L, bits) <= s.cap) {
     keyset_dedup(L, in, n, bits, swap, full, full ? n_full : 0, head, n_head, out, d_nout, s);
     return;

@@ -54,6 +54,18 @@ def test_sort_unique_one_digit(n):
                         oracle.sort_unique(keys_with_bits(np.random.default_rng(n), n, 7)))
 
 
+@pytest.mark.parametrize('bits,n', [(17, 100), (17, 5003), (32, 16_384), (5, 300_000), (13, 3_000_000), (16, 20_000)])
+def test_sort_unique_refuses_little_scratch(bits, n):
+  '''A region for the packed keys alone is too small, whichever path they take.'''
+  k = torch.from_numpy(keys_with_bits(np.random.default_rng(n), n, bits).view(np.int64)).cuda()
+  out, d_n = torch.full_like(k, -1), torch.full((1,), -1, dtype=torch.int64, device='cuda')
+  size = 2 * n * (4 if bits <= 16 else 8)
+  scratch = torch.empty(size, dtype=torch.uint8, device='cuda')
+  rc = native.lib().srdl_sort_unique_u64(k.data_ptr(), n, bits, out.data_ptr(), d_n.data_ptr(), scratch.data_ptr(),
+                                         size, torch.cuda.current_stream().cuda_stream)
+  assert rc == 5 and int(d_n) == -1 and bool((out == -1).all())
+
+
 @pytest.mark.parametrize('na,nb', [(1, 4), (2047, 2049), (2048, 2048), (31, 6000), (4096, 4096 * 16),
                                    (4096, 4096 * 16 + 1), (20_481, 700_000), (1_300_000, 2),
                                    # both sides of the line between streaming FULL and searching it
