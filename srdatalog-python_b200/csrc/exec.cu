@@ -15,9 +15,9 @@
 #include <chrono>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
 #include <mutex>
 #include <sstream>
-#include <system_error>
 #include <thread>
 
 #include "runtime.h"
@@ -1133,7 +1133,10 @@ void Database::copy_rows(const uint64_t* keys, uint64_t n, int arity, uint32_t* 
     pieces = (n + per - 1) / per;
     T = 1;
   }
-  std::vector<Error> errs((size_t)T, Error{0, ""});
+  // (no exception leaves a thread, and none is thrown here while one runs)
+  std::vector<std::exception_ptr> errs((size_t)T);
+  std::vector<std::thread> threads;
+  threads.reserve((size_t)T);
   auto work = [&](int t) {
     cudaEvent_t ev = nullptr;
     try {
@@ -1147,23 +1150,22 @@ void Database::copy_rows(const uint64_t* keys, uint64_t n, int arity, uint32_t* 
         SRDL_CUDA(cudaEventSynchronize(ev));
         memcpy(dst + r0 * row, stage, cnt * row);
       }
-    } catch (const Error& e) {
-      errs[t] = e;
+    } catch (...) {
+      errs[t] = std::current_exception();
     }
     if (ev) cudaEventDestroy(ev);
   };
-  std::vector<std::thread> threads;
   int started = 1;
   try {
     for (; started < T; started++) threads.emplace_back(work, started);
-  } catch (const std::system_error&) {
-    // no more threads: this one does the rest
+  } catch (const std::exception&) {
+    // no more threads (or no memory for one): this one does the rest
   }
   work(0);
   for (auto& t : threads) t.join();
   for (int t = started; t < T; t++) work(t);
   for (auto& e : errs)
-    if (e.code) throw e;
+    if (e) std::rethrow_exception(e);
 }
 
 std::string Database::stats_json() const {
