@@ -84,9 +84,9 @@ int srdl_set_profiling(srdl_db* db, int enable);
  *   "lsm_compact_pct"  Device2LevelIndex: merge HEAD into FULL once HEAD
  *                      exceeds this percentage of FULL (default 10, the
  *                      reference's kCompactRatio, device_2level_index.h:300)
- *   "radix_bits"       widest radix-sort digit, 1..8: a sort of b-bit keys
- *                      runs ceil(b / radix_bits) passes; 8 (default) leaves
- *                      the width to the sort, which takes 9 bits
+ *   "radix_bits"       widest radix-sort digit, 1..8: a sort of b-bit keys by
+ *                      counting passes runs ceil(b / radix_bits); 8 (default)
+ *                      leaves the width to the sort, which takes 9 bits
  *   "join_blocks_per_sm"  join launches use at most this many blocks per
  *                      SM, 1..64 (default 16): the candidates per warp
  *   "join_chunk"       largest chunk of candidates a warp of the two-source
@@ -95,8 +95,8 @@ int srdl_set_profiling(srdl_db* db, int enable);
  *   "pivot_min"        count-only two-source joins: rows whose list of the
  *                      table's first (sorted) column has at least this many
  *                      values are counted by a kernel that holds the list as
- *                      a bitmap in shared memory (0: never; unset: 256 for
- *                      tables of at least 2^20 rows)
+ *                      a bitmap in shared memory (0: never; -1, the default:
+ *                      256 for tables of at least 2^20 rows)
  *   "device_loop"      1 (default; SRDL_DEVICE_LOOP=0 changes it) runs the
  *                      iterations of a qualifying recursive step after the
  *                      first as one CUDA graph that loops on the device

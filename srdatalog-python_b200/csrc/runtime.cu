@@ -944,7 +944,8 @@ static uint32_t hash_min_len() {
 }
 
 void Database::set_option(const std::string& name, int64_t value) {
-  SRDL_REQUIRE(value >= 0, kErrArg, "set_option: negative value for " + name);
+  SRDL_REQUIRE(value >= 0 || (value == -1 && name == "pivot_min"), kErrArg,
+               "set_option: negative value for " + name);
   if (name == "bitmap_mb") opt_bitmap_mb_ = value;
   else if (name == "hash_min") opt_hash_min_ = value;
   else if (name == "lsm_compact_pct") opt_lsm_pct_ = value;
@@ -965,7 +966,7 @@ void Database::set_option(const std::string& name, int64_t value) {
     SRDL_REQUIRE(value >= 1 && value <= 64, kErrArg, "set_option: join_blocks_per_sm out of [1, 64]");
     L_.join_bpsm = (int)value;
   } else if (name == "pivot_min") {
-    SRDL_REQUIRE(value >= 0 && value <= (1ll << 32), kErrArg, "set_option: pivot_min out of [0, 2^32]");
+    SRDL_REQUIRE(value <= (1ll << 32), kErrArg, "set_option: pivot_min out of [-1, 2^32]");
     opt_pivot_min_ = value;
   }
   else throw Error{kErrArg, "set_option: unknown option " + name};

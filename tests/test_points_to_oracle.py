@@ -128,3 +128,13 @@ def test_set_option_rejects_unknown_names():
     with pytest.raises(Exception):
       db.set_option(name, bad)
   db.close()
+
+
+def test_pivot_min_takes_its_default_back():
+  from srdatalog_b200 import native
+  with native.Database(load_plan('triangle')) as db:
+    for v in (0, 1 << 32, -1):
+      db.set_option('pivot_min', v)
+    for v in (-2, (1 << 32) + 1):
+      with pytest.raises(native.SrdlError):
+        db.set_option('pivot_min', v)
