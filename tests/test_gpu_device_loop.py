@@ -4,6 +4,8 @@ give the host path's results -- bit-exact against the oracle and the golden
 fixtures -- including when too-small capacities send iterations back to the
 host path (overflow), under max_iters, and on repeated runs.'''
 
+import copy
+
 import numpy as np
 import oracle
 import pytest
@@ -14,9 +16,13 @@ from srdatalog_b200 import workloads as W
 pytestmark = pytest.mark.gpu
 
 
-def run(plan, inputs, loop=True, cap=0, max_iters=0, repeat=1):
-  db = native.Database(load_plan(plan))
+def run(plan, inputs, loop=True, cap=0, max_iters=0, repeat=1, sets=True):
+  '''sets=False: a memory limit far above the run's need, under which NEW and
+  FULL are sorted arrays also where bitmap sets would be taken.'''
+  db = native.Database(load_plan(plan) if isinstance(plan, str) else plan)
   db.set_option('device_loop', 1 if loop else 0)
+  if not sets:
+    db.set_option('mem_limit_mb', 1 << 16)
   if cap:
     db.set_option('device_loop_cap_limit', cap)
   for rel, rows in inputs.items():
@@ -76,13 +82,15 @@ def test_tc_variants_equal_host_path_and_oracle(plan, n, m, seed):
   assert dev.size('Path') == keys.shape[0]
 
 
-@pytest.mark.parametrize('cap', [1024, 4096, 20_000])
-def test_overflow_hands_iterations_back_to_the_host(cap, expected):
+@pytest.mark.parametrize('sets', [True, False])
+@pytest.mark.parametrize('cap', [1024, 4096, 20_000, 300_000])
+def test_overflow_hands_iterations_back_to_the_host(cap, sets, expected):
   '''Capacities far below the counts: kernels raise the overflow flag
   instead of writing past a buffer, the loop stops, the failed iteration is
-  redone on the host path from the intact buffer set, and the loop is
-  entered again; the result is still the golden one.'''
-  db = run('tc', {'ArcInput': W.tc_small(1)}, cap=cap)
+  redone on the host path from what it read (the other buffer set; with bitmap
+  sets, unchanged), and the loop is entered again; the result is still the
+  golden one.'''
+  db = run('tc', {'ArcInput': W.tc_small(1)}, cap=cap, sets=sets)
   st = loop_stats(db)
   assert st['overflows'] >= 1, st
   assert db.size('Path') == expected['tc_small']['size']
@@ -102,6 +110,70 @@ def test_no_room_for_the_final_full():
   same(db, run('tc', {'ArcInput': e}, loop=False), 'Path')
   assert db.size('Path') == 600 * 601 // 2
   assert rec_iterations(db) == [600]
+
+
+def odd_even_plan():
+  '''Two relations computed by one recursive step: Path holds the pairs joined
+  by an odd number of edges, Even those by an even one.'''
+  plan = load_plan('tc')
+  path = next(r for r in plan['relations'] if r['name'] == 'Path')
+  plan['relations'].append(dict(path, name='Even'))
+
+  def renamed(ops, to):
+    out = copy.deepcopy(ops)
+    for o in out:
+      if o.get('rel') == 'Path':
+        o['rel'] = to
+    return out
+
+  rec = next(s for s in plan['steps'] if s['recursive'])
+  rule, rest = rec['ops'][0], rec['ops'][1:]
+  rules = []
+  for src, dst in (('Path', 'Even'), ('Even', 'Path')):
+    r = copy.deepcopy(rule)
+    r['rule'] = 'To' + dst
+    for po in r['pipeline'][:2]:
+      po['sources'][0]['rel'] = src
+    r['pipeline'][2]['rel'] = dst
+    rules.append(r)
+  rec['ops'] = rules + rest + renamed(rest, 'Even')
+  last = plan['steps'][-1]
+  last['ops'] = last['ops'] + renamed(last['ops'], 'Even')
+  return plan
+
+
+@pytest.mark.parametrize('sets', [True, False])
+@pytest.mark.parametrize('cap', [0, 2000, 9000, 40_000])
+def test_overflow_of_a_step_that_computes_two_relations(cap, sets):
+  '''One relation's delta outgrows its capacity while the other's fits: neither
+  is changed in that iteration.'''
+  n = 700
+  e = W.uniform_edges(n, 1500, 5)
+  db = run(odd_even_plan(), {'ArcInput': e}, cap=cap, sets=sets, repeat=2 if not cap else 1)
+  st = loop_stats(db)
+  assert st['entries'] >= 1 and (st['overflows'] >= 1) == (cap > 0), st
+  d = np.concatenate([np.stack([e[:, 0], e[:, 1] + n], 1), np.stack([e[:, 0] + n, e[:, 1]], 1)])
+  pairs = oracle.unpack(oracle.tc(d.astype(np.uint32))[0], order=(1, 0))
+  pairs = pairs[pairs[:, 0] < n]   # paths from the even copy of x
+  odd = pairs[:, 1] >= n
+  for rel, want in (('Path', pairs[odd] - np.array([0, n], np.uint32)), ('Even', pairs[~odd])):
+    assert db.size(rel) == want.shape[0] > 0, rel
+    assert db.hash(rel) == oracle.dump_hash(want), rel
+  host = run(odd_even_plan(), {'ArcInput': e}, loop=False)
+  assert rec_iterations(db) == rec_iterations(host)
+
+
+@pytest.mark.parametrize('sets', [True, False])
+@pytest.mark.parametrize('max_iters', [2, 3, 4, 5, 6, 9])
+def test_max_iters_on_either_representation(max_iters, sets):
+  '''The loop stops at odd and at even iterations, with values of 11 bits (NEW
+  and FULL as bitmap sets) and of 16 (as sorted arrays).'''
+  e = W.uniform_edges(2000, 6000, 7) * np.uint32(1 if sets else 30)
+  dev = run('tc', {'ArcInput': e}, max_iters=max_iters, repeat=2)
+  host = run('tc', {'ArcInput': e}, loop=False, max_iters=max_iters)
+  assert loop_stats(dev)['iterations'] == max_iters - 1
+  same(dev, host, 'Path')
+  assert rec_iterations(dev) == rec_iterations(host) == [max_iters]
 
 
 @pytest.mark.parametrize('max_iters', [1, 2, 3, 5, 9])

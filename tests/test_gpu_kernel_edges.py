@@ -27,17 +27,20 @@ def test_sort_unique_block_edges(n, bits):
 
 
 # a bitmap set sorts when the key space has at most 4,096 keys per input key and
-# at most 2^28 in all
-@pytest.mark.parametrize('bits,n', [(1, 16_385), (5, 20_000), (6, 20_000), (13, 16_385), (14, 65_535), (14, 65_536),
-                                    (14, 3_000_000), (15, 3_000_000)])
+# at most 2^28 in all, and the caller's scratch has room for it (33 MB at most);
+# with the stated scratch it has that for small sets or many keys
+@pytest.mark.parametrize('room', [0, 40 << 20])
+@pytest.mark.parametrize('bits,n', [(1, 16_385), (5, 6001), (5, 20_000), (6, 20_000), (12, 6000), (12, 6001),
+                                    (13, 16_384), (13, 16_385), (14, 65_535), (14, 65_536), (14, 3_000_000),
+                                    (15, 3_000_000)])
 @pytest.mark.parametrize('dense', [False, True])
-def test_sort_unique_key_sets(bits, n, dense):
+def test_sort_unique_key_sets(bits, n, dense, room):
   rng = np.random.default_rng(n + bits)
   k = keys_with_bits(rng, n, bits)
   if dense:   # a block of the key space filled, the rest nearly empty
     k[: n - n // 16] = keys_with_bits(rng, n - n // 16, max(1, bits - 3))
   k[n // 2] = ((1 << bits) - 1) << 32 | ((1 << bits) - 1)
-  assert np.array_equal(gpu_sort_unique(k, bits), oracle.sort_unique(k))
+  assert np.array_equal(gpu_sort_unique(k, bits, room=room), oracle.sort_unique(k))
 
 
 @pytest.mark.parametrize('n', [5000, 300_000])

@@ -29,13 +29,14 @@ def stream():
   return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
-def gpu_sort_unique(keys, bits, alias=False):
+def gpu_sort_unique(keys, bits, alias=False, room=0):
+  '''room: scratch bytes, where that is more than the sort states.'''
   lib = native.lib()
   n = len(keys)
   d_in = dev(keys)
   d_out = d_in if alias else torch.empty(max(n, 1), dtype=torch.int64, device='cuda')
   d_n = torch.full((1,), -1, dtype=torch.int64, device='cuda')
-  sb = lib.srdl_sort_unique_scratch_bytes(n, bits)
+  sb = max(lib.srdl_sort_unique_scratch_bytes(n, bits), room)
   scratch = torch.empty(max(sb, 1), dtype=torch.uint8, device='cuda')
   rc = lib.srdl_sort_unique_u64(d_in.data_ptr(), n, bits, d_out.data_ptr(), d_n.data_ptr(),
                                 scratch.data_ptr(), sb, stream())

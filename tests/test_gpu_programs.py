@@ -433,6 +433,22 @@ def test_tuning_options_keep_results(expected, radix_bits, jbpsm):
   assert t.count('TriangleJoin') == expected['triangle_rmat14']['count']
 
 
+@pytest.mark.parametrize('radix_bits', range(1, 9))
+@pytest.mark.parametrize('top', [40_000, 1_000_003])
+def test_radix_bits_on_counting_passes(radix_bits, top):
+  '''Relations that are sorted by counting passes (more than 16,384 rows, values
+  past 14 bits), with digits of every width; 32- and 64-bit packed keys.'''
+  e = np.random.default_rng(top).integers(0, top, (50_001, 2)).astype(np.uint32)
+  e[0] = top - 1, top - 1
+  with native.Database(load_plan('triangle')) as db:
+    db.set_option('radix_bits', radix_bits)
+    db.load_rows('KnowsInput', np.concatenate([e, e[::3]]))
+    db.run()
+    want = np.unique(e, axis=0)
+    assert np.array_equal(db.dump('Knows'), want)
+    assert db.count('TriangleJoin') == oracle.triangle_count(want)
+
+
 @pytest.mark.parametrize('bits,m,keys', [(17, 9000, 'one block'), (13, 90_000, 'set'), (15, 60_000, 'passes'),
                                          (18, 60_000, 'passes')])
 def test_sort_bytes(bits, m, keys):
