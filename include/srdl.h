@@ -255,7 +255,9 @@ int srdl_sha256(const void* data, uint64_t n_bytes, unsigned char* out32);
  * temporaries live in the caller's scratch region.
  * ---------------------------------------------------------------------- */
 
-/* Scratch bytes srdl_sort_unique_u64 needs for n keys. */
+/* Scratch bytes srdl_sort_unique_u64 needs for n keys.  With values below 2^14
+ * a region that also holds one bit per possible key and 1 MB (33 MB at most) is
+ * used for such a bitmap where that sorts faster. */
 uint64_t srdl_sort_unique_scratch_bytes(uint64_t n, int value_bits);
 
 /* Sort n keys ascending and drop duplicates: d_out gets the distinct keys,

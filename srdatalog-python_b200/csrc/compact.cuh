@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(kCpThreads) cp_write_kernel(Sel sel, uint64_t 
   }
 }
 
-// Runs the three launches; the selected count lands in *d_total.  With d_n,
+// Runs the two launches; the selected count lands in *d_total.  With d_n,
 // n is a capacity and the element count is *d_n (device loop).
 template <class Sel>
 void compact(const Launch& L, Sel sel, uint64_t n, uint64_t* d_total, Scratch& s,
@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(kCpThreads) dd_probe_kernel(DedupDiffSel<K, PL
 // tiles of kCpTile elements (one thread per tile boundary finds the cut by
 // merge-path binary search, and the tile's start in HEAD).  Persistent blocks
 // walk the tiles; the next tile's two slices are copied into the second
-// shared buffer with cp.async while the current tile is merged, 8 merged
+// shared buffer with cp.async while the current tile is merged, 16 merged
 // elements per thread.  An a-key is kept iff it differs from the last FULL
 // key taken at or before it (so it is not in FULL) and from the a-key before
 // it (dedup); HEAD, when present, is probed per kept key within the tile's

@@ -10,9 +10,9 @@
 // coalesced.
 //
 // set_difference replaces thrust::set_difference on the zipped columns
-// (.ipp:1104-1107) and the binary-probe variant (.ipp:933-1041): every
-// element of `a` is probed in the slice of `b` that its block's key range
-// can reach, then the survivors are compacted in order.
+// (.ipp:1104-1107) and the binary-probe variant (.ipp:933-1041): `a` and `b` are
+// merged tile by tile, or every element of `a` is searched in `b` (compact.cuh),
+// then the survivors are compacted in order.
 #include <algorithm>
 #include <atomic>
 

@@ -10,7 +10,8 @@ None of the knobs changes a result; they trade memory and work:
   indexes (0 turns them off);
 * ``lsm_compact_pct``: HEAD is merged into FULL once it exceeds this
   percentage of FULL (only tried when some relation uses the LSM policy);
-* ``radix_bits``: widest radix-sort digit (passes = key bits / this);
+* ``radix_bits``: widest radix-sort digit (passes = key bits / this; 8, the
+  default, leaves the width to the sort, which takes 9);
 * ``join_blocks_per_sm``: grid cap of the join launches, i.e. the
   candidates each warp walks (the work-splitting chunk).
 

@@ -153,8 +153,8 @@ def test_merge_disjoint(na, nb):
 
 
 def test_sort_unique_many_tiles():
-  '''20M keys of 2 x 21 bits: six 7-bit passes over ~10K tiles spread over
-  every block of the grid.'''
+  '''20M keys of 2 x 21 bits: five passes of 8 and 9 bits over ~2,400 tiles, several
+  of them for every block of the grid.'''
   rng = np.random.default_rng(11)
   k = keys_with_bits(rng, 20_000_000, 21, dup_frac=0.1)
   assert np.array_equal(gpu_sort_unique(k, 21), oracle.sort_unique(k))
