@@ -286,18 +286,19 @@ int Database::run_device_loop(const Step& st, uint64_t it0, uint64_t max_iters, 
                               (sets ? 2 * set_bytes + lr.cap_full * 8
                                     : lr.cap_new * 8 + lr.cap_full * 16 +
                                           sort_dev_scratch_bytes(lr.cap_new, lr.cap_full, bits_));
-        // (asked only when the arena's cached blocks, which a run before this one
-        // has left, are fewer: the query waits for whoever else talks to the
-        // driver -- with nvidia-smi sampling beside it a TC step of 2.6 ms took
-        // up to 59 ms, all of it here)
+        // (asked only for more than the arena has cached and than an earlier run
+        // was granted, whose blocks the arena keeps: the query waits for whoever
+        // else talks to the driver -- a TC step of 2.6 ms took up to 59 ms, all of
+        // it here)
         const ArenaUse au = arena_use(L_.stream);
-        if (need > au.cached) {
+        if (need > std::max<uint64_t>(au.cached, loop_granted_)) {
           size_t free_b = 0, total_b = 0;
           SRDL_CUDA(cudaMemGetInfo(&free_b, &total_b));
           if ((double)need > 0.7 * (double)(free_b + au.cached))
             throw Error{kErrCapacity, "device loop buffers (" + std::to_string(need >> 20) +
                                           " MB) would take most of the free device memory"};
         }
+        loop_granted_ = std::max(loop_granted_, need);
       }
       if (!sets) lr.newk = DevBuf(lr.cap_new * 8, L_.stream);
       if (sets) {

@@ -315,6 +315,7 @@ class Database {
   // Frees the blocks this database's stream arena caches for reuse.
   void trim_cache() {
     if (dev_ready_) arena_trim(L_.stream);
+    loop_granted_ = 0;
   }
   bool any_loaded() const;
   void stage_facts(Relation& r);
@@ -400,6 +401,7 @@ class Database {
   // across runs: the device loop sizes its buffers from them.
   std::map<const Op*, std::vector<uint64_t>> level_max_;
   std::map<std::string, uint64_t> new_max_, delta_max_, full_max_;
+  uint64_t loop_granted_ = 0;  // most bytes of a relation's loop buffers that the device had room for
   size_t prof_begin(const std::string& name);
   void prof_end(size_t id, double bytes, double units);
   void prof_collect();
