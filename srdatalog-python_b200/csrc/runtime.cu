@@ -1004,9 +1004,10 @@ void Database::ensure_hash(Index& ix) {
 // dependent steps.  The threshold is the smallest length kBitmapMinLen * 2^k
 // whose bitmaps (one bit per value of the domain each) fit in SRDL_BITMAP_MB
 // (default 768 MB; 0 disables); domains above 2^24 values get none.  On the
-// R-MAT scale-20 triangle count the default picks lists of 512 or more
-// (4,552 bitmaps, 569 MB): 14.1 ms per step, against 14.8 ms at 1,024,
-// 16.1 ms at 2,048 and 14.2-14.4 ms at 256 and 128.
+// R-MAT scale-20 triangle count, whose longest lists the pivot kernel holds in
+// shared memory instead, the default picks lists of 512 or more (4,552 bitmaps,
+// 569 MB): 7.33 ms per step, against 7.34 / 7.42 / 7.41 / 7.63 ms with budgets of
+// 512 / 256 / 128 / 64 MB, 7.47 with 2,048 and 8.20 with none.
 static uint64_t bitmap_budget() {
   static const uint64_t v = [] {
     const char* e = getenv("SRDL_BITMAP_MB");
